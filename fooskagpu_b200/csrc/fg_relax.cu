@@ -17,254 +17,321 @@ namespace fg {
 
 namespace {
 
-struct Ph {
-    double g, pinf, cp, eta;
-};
-
-__device__ __forceinline__ double p_of(const Ph &h, double r, double e) {
-    return (h.g - 1) * r * e - h.g * h.pinf - (h.g - 1) * h.eta * r;
+// pressure and temperature of phase m at density r and internal energy e (DP/eqos.h); the phase
+// constants are precomputed once per launch (RelaxParams)
+__device__ __forceinline__ double p_of(const RelaxParams &R, int m, double r, double e) {
+    return R.gm1[m] * r * e - R.gpinf[m] - R.gm1eta[m] * r;
 }
-__device__ __forceinline__ double t_of(const Ph &h, double r, double e) {
-    const double p = (h.g - 1) * r * e - h.g * h.pinf - (h.g - 1) * h.eta * r;
-    return (p + h.pinf) / ((h.cp / h.g) * (h.g - 1) * r);
+__device__ __forceinline__ double t_of(const RelaxParams &R, int m, double r, double e) {
+    return (p_of(R, m, r, e) + R.pinf[m]) / (R.cvgm1[m] * r);
 }
 
+// log10(1 + d) for |d| < kSmallLog by the Taylor series of the logarithm, truncated below 1e-18 of
+// the value: the forward differences of the Newton solves change the argument of a logarithm by
+// 1e-3 .. 1e-8 of itself, and the series gives that change directly, without the cancellation of
+// two logarithms and at a tenth of the cost of the second one
+constexpr double kLog10e = 0.43429448190325182765, kSmallLog = 1e-3;
+__device__ __forceinline__ double log10_1p(double d) {
+    const double s = 1.0 + d * (-1.0 / 2 + d * (1.0 / 3 + d * (-1.0 / 4 + d * (1.0 / 5 + d * (-1.0 / 6)))));
+    return (kLog10e * d) * s;
+}
+
+// Newton on the saturation temperature (DP/relaxation.cu:4-38) with the reference's forward
+// difference dT = 1e-3 K.  The difference f(T + dT) - f(T) of f = A + B / T + C log10 T comes from the
+// series in d = dT / T, so an iteration takes one logarithm and two divisions (partition of the 981 k-tet
+// bubble: 66 -> 43 us; of the jet, most of whose cells are below chemLimit and skip it: 122 -> 12 us).
 __device__ double sat_temp(const RelaxParams &R, double P, double temp, double urf) {
-    const double Pinf = R.pinf[0];
-    const double g1 = R.gam[0], g2 = R.gam[1];
-    const double Cp1 = R.cp[0], Cp2 = R.cp[1];
-    const double Cv1 = Cp1 / g1, Cv2 = Cp2 / g2;
     const double etaT2 = R.satConst[0] * log10(P) + R.satConst[1];
-    const double As = (Cp1 - Cp2 + etaT2 - 0.0) / (Cp2 - Cv2);
-    const double Bs = (R.eta[0] - R.eta[1]) / (Cp2 - Cv2);
-    const double Cs = (Cp2 - Cp1) / (Cp2 - Cv2);
-    const double Ds = (Cp1 - Cv1) / (Cp2 - Cv2);
     const double dT = 1.e-3;
-    const double lpp = Ds * log10(P + Pinf), lp = log10(P);
+    const double rest = (R.satA + etaT2) * R.satQ + R.satD * log10(P + R.pinf[0]) - log10(P);
     double fun = 1, T = temp;
     for (int itr = 0; fabs(fun) > 1.e-2 && itr < 50; itr++) {
-        fun = As + Bs / T + Cs * log10(T) + lpp - lp;
-        const double fdt = As + Bs / (T + dT) + Cs * log10(T + dT) + lpp - lp;
-        T = T - urf * fun / ((fdt - fun) / dT);
+        const double iT = 1.0 / T, d = dT * iT;
+        fun = rest + R.satB * iT + R.satC * log10(T);
+        double df;
+        if (fabs(d) < kSmallLog) {
+            // 1 / (T + dT) - 1 / T = -(1 / T) d (1 - d + d^2 - ...)
+            df = R.satC * log10_1p(d) - R.satB * iT * d * (1.0 - d * (1.0 - d * (1.0 - d * (1.0 - d * (1.0 - d)))));
+        } else {
+            df = R.satB / (T + dT) - R.satB * iT + R.satC * (log10(T + dT) - log10(T));
+        }
+        T = T - urf * fun * dT / df;
     }
     return T;
 }
 
-__device__ __forceinline__ void therm_res(const Ph *h, int pm, double *x, const double *ar, const double *enr,
-                                          double *r0, double *r1) {
-    const int mm = 1 - pm;
-    const double s1 = ar[mm] / x[mm];
-    const double s2 = ar[mm] * (x[2 + mm] - enr[mm]);
-    x[pm] = (1 / (1 - s1)) * ar[pm];
-    x[2 + pm] = enr[pm] - (1 / ar[pm]) * s2;
-    *r0 = p_of(h[0], x[0], x[2]) - p_of(h[1], x[1], x[3]);
-    *r1 = t_of(h[0], x[0], x[2]) - t_of(h[1], x[1], x[3]);
-}
-
-__device__ int therm_cell(const RelaxParams &R, const Ph *h, double *U, int *iters) {
-    double ar[2], enr[2], x[4], ax[4];
+// Thermal (p, T) equilibrium (DP/thermRlx.cu:4-235).  The unknowns are the density r and energy e of
+// the minor phase; the primary phase follows from volume and energy.  The two solved phases are
+// named minor / primary and mapped to the phases 0 / 1 by selects, so no array is indexed at run
+// time; the energy difference reuses the densities and their reciprocals, and each iteration takes
+// 11 divisions where the reference's order of operations takes 23 (981 k-tet bubble, 8.6 iterations
+// per cell: 255 -> 162 us; 2.0 M-cell jet: 241 -> 158 us).
+__device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
     const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
     const double a1 = 1 - a0;
     const double rho0 = U[1] / a0, rho1 = U[2] / a1;
-    ar[0] = a0 * rho0;
-    ar[1] = a1 * rho1;
-    enr[0] = U[6] / ar[0];
-    enr[1] = U[7] / ar[1];
-    const double rm = ar[0] + ar[1];
-    const double u = U[3] / rm, v = U[4] / rm, w = U[5] / rm;
-    x[0] = rho0; x[1] = rho1; x[2] = enr[0]; x[3] = enr[1];
-#pragma unroll
-    for (int i = 0; i < 4; i++) ax[i] = x[i];
-    const int pm = (a1 > a0) ? 1 : 0;
-    const double de = U[8] / rm - (ar[0] / rm) * enr[0] - (ar[1] / rm) * enr[1] - 0.5 * (u * u + v * v + w * w);
-    enr[0] += de;
-    enr[1] += de;
-    const int mm = 1 - pm;
+    const double ar0 = a0 * rho0, ar1 = a1 * rho1;
+    const double e0 = U[6] / ar0, e1 = U[7] / ar1;
+    const bool m1 = !(a1 > a0);   // the minor phase is phase 1
+    const double arm = m1 ? ar1 : ar0, arp = m1 ? ar0 : ar1;
+    double r = m1 ? rho1 : rho0, e = m1 ? e1 : e0;
+    double enm, enp;
+    {
+        const double im = 1.0 / (ar0 + ar1);
+        const double u = U[3] * im, v = U[4] * im, w = U[5] * im;
+        const double de = U[8] * im - (ar0 * im) * e0 - (ar1 * im) * e1 - 0.5 * (u * u + v * v + w * w);
+        enm = e + de;
+        enp = (m1 ? e0 : e1) + de;
+    }
+    const double iarp = 1.0 / arp;
+    double br = r, be = e;   // best iterate
     float minRes = 1e9f;
-    int abortFlag = 0, aborted = 0;
+    int aborted = 0;
     for (int itr = 1;; itr++) {
         *iters = itr;
-        double res[2], rdf[2][2], e[2];
-        therm_res(h, pm, x, ar, enr, &res[0], &res[1]);
-        // finite-difference Jacobian over the minor phase's (rho, e)
-        const int js[2] = {mm, mm + 2};
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int j = js[q];
-            e[q] = 1e-4 * x[j];
-            x[j] += e[q];
-            therm_res(h, pm, x, ar, enr, &rdf[0][q], &rdf[1][q]);
-            x[j] -= e[q];
+        // residuals at (r, e)
+        double rp = arp / (1 - arm / r);
+        const double ep = enp - iarp * (arm * (e - enm));
+        const double i0 = 1.0 / (R.cvgm1[0] * (m1 ? rp : r)), i1 = 1.0 / (R.cvgm1[1] * (m1 ? r : rp));
+        double p0 = p_of(R, 0, m1 ? rp : r, m1 ? ep : e), p1 = p_of(R, 1, m1 ? r : rp, m1 ? e : ep);
+        const double res0 = p0 - p1, res1 = (p0 + R.pinf[0]) * i0 - (p1 + R.pinf[1]) * i1;
+        const bool inside = r > 0.0 && rp > 0.0;
+        // forward differences in e (same densities), then in r (same energies)
+        const double he = 1e-4 * e, hr = 1e-4 * r;
+        double j01, j11, j00, j10;
+        {
+            const double eq = e + he, epq = enp - iarp * (arm * (eq - enm));
+            p0 = p_of(R, 0, m1 ? rp : r, m1 ? epq : eq);
+            p1 = p_of(R, 1, m1 ? r : rp, m1 ? eq : epq);
+            const double ih = 1.0 / he;
+            j01 = ((p0 - p1) - res0) * ih;
+            j11 = (((p0 + R.pinf[0]) * i0 - (p1 + R.pinf[1]) * i1) - res1) * ih;
         }
-        double jac[2][2];
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                jac[i][j] = (rdf[i][j] - res[i]) / e[j];
-                if (isnan(jac[i][j])) abortFlag = 1;
-            }
-        const double det = jac[0][0] * jac[1][1] - jac[1][0] * jac[0][1];
-        const double i00 = jac[1][1] / det, i11 = jac[0][0] / det, i10 = -jac[1][0] / det, i01 = -jac[0][1] / det;
-        if (det == 0) abortFlag = 1;
-        if (abortFlag == 0 && x[0] > 0.0 && x[1] > 0.0) {
-            const float chk = sqrt(res[0] * res[0] + res[1] * res[1]);
+        {
+            const double rq = r + hr;
+            rp = arp / (1 - arm / rq);
+            const double x0 = m1 ? rp : rq, x1 = m1 ? rq : rp;
+            p0 = p_of(R, 0, x0, m1 ? ep : e);
+            p1 = p_of(R, 1, x1, m1 ? e : ep);
+            const double ih = 1.0 / hr;
+            j00 = ((p0 - p1) - res0) * ih;
+            j10 = (((p0 + R.pinf[0]) / (R.cvgm1[0] * x0) - (p1 + R.pinf[1]) / (R.cvgm1[1] * x1)) - res1) * ih;
+        }
+        const double det = j00 * j11 - j10 * j01;
+        const bool bad = isnan(j00) || isnan(j01) || isnan(j10) || isnan(j11) || det == 0;
+        if (!bad && inside) {
+            const float chk = sqrt(res0 * res0 + res1 * res1);
             if (chk < minRes) {
                 minRes = chk;
-#pragma unroll
-                for (int i = 0; i < 4; i++) ax[i] = x[i];
+                br = r;
+                be = e;
             }
         }
-        x[mm] = x[mm] - R.thermUrf * (i00 * res[0] + i01 * res[1]);
-        x[mm + 2] = x[mm + 2] - R.thermUrf * (i10 * res[0] + i11 * res[1]);
-        const bool conv = !(fabs(res[0]) > 1.e-2) && !(fabs(res[1]) > 1.e-2);
-        if (abortFlag == 1 || itr > R.thermItrMax) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) x[i] = ax[i];
+        if (bad || itr > R.thermItrMax) {
+            r = br;
+            e = be;
             aborted = 1;
             break;
         }
-        if (conv) break;
+        const double id = R.thermUrf / det;
+        r = r - id * (j11 * res0 - j01 * res1);
+        e = e - id * (j00 * res1 - j10 * res0);
+        if (!(fabs(res0) > 1.e-2) && !(fabs(res1) > 1.e-2)) break;
     }
-    const double s1 = ar[mm] / x[mm];
-    const double s2 = ar[mm] * (x[2 + mm] - enr[mm]);
-    x[pm] = (1 / (1 - s1)) * ar[pm];
-    x[2 + pm] = enr[pm] - (1 / ar[pm]) * s2;
-    U[0] = fmin(fmax(R.avfMin / 100, ar[0] / x[0]), 1 - R.avfMin / 100);
-    U[6] = ar[0] * x[2];
-    U[7] = ar[1] * x[3];
+    const double rp = arp / (1 - arm / r);
+    const double ep = enp - iarp * (arm * (e - enm));
+    U[0] = fmin(fmax(R.avfMin / 100, ar0 / (m1 ? rp : r)), 1 - R.avfMin / 100);
+    U[6] = ar0 * (m1 ? ep : e);
+    U[7] = ar1 * (m1 ? e : ep);
     return aborted;
 }
 
-__device__ __forceinline__ double gibbs_of(const RelaxParams &R, int m, double P, double T) {
-    const double et = (m == 1) ? R.satConst[0] * log10(P) + R.satConst[1] : 0.0;
-    const double hh = R.cp[m] * T + R.eta[m];
-    const double s = (R.cp[m] / R.gam[m]) * log10(pow(T, R.gam[m]) / pow(P + R.pinf[m], R.gam[m] - 1)) + et;
-    return hh - T * s;
+// Residuals of the chemical (p, T, Gibbs) equilibrium of a cell with mixture density rm and internal
+// energy re per unit volume (DP/chemRlx.cu:4-130), and their forward-difference Jacobian.  The
+// unknowns are volume fraction a, density r and energy e of the minor phase (phase 1 if m1).
+// The reference's entropy log10(T^g / (p + pinf)^(g - 1)) is evaluated as g log10 T - (g - 1)
+// log10(p + pinf), with no powers; the logarithms are taken once, at the base point, and the three
+// perturbed points add log10 of the ratio from the series (log10_1p), or logarithms of their own
+// where the ratio is not near 1: 4 logarithms an iteration in place of 12 and 16 powers.  Bound by FP64
+// instructions (and, on few cells, by the latency of one cell's chain of iterations): the relaxation
+// kernel went 784 -> 241 us on a 61 x 67 x 59 box with 36 % chemical cells, 331 -> 130 us on 16,096 cells
+// of mixed elements, and 387 -> 119 us on a 64^3 box with the surrogate's polish.
+struct ChemLog {
+    double lT[2], lP[2], lG;   // log10 of T, p + pinf of the phases, and of the gas pressure
+};
+struct ChemSystem {
+    double res[3], jac[3][3];
+    double ap, rp;   // volume fraction and density of the primary phase at the base point
+    // the base point: pressures, temperatures, reciprocals of T and p + pinf, logarithms
+    double p[2], T[2], iT[2], iP[2];
+    ChemLog log;
+};
+__device__ __forceinline__ double chem_gibbs_diff(const RelaxParams &R, const double *T, const ChemLog &l) {
+    const double s0 = R.cv[0] * (R.gam[0] * l.lT[0] - R.gm1[0] * l.lP[0]);
+    const double s1 = R.cv[1] * (R.gam[1] * l.lT[1] - R.gm1[1] * l.lP[1]) + (R.satConst[0] * l.lG + R.satConst[1]);
+    return (R.cp[0] * T[0] + R.eta[0] - T[0] * s0) - (R.cp[1] * T[1] + R.eta[1] - T[1] * s1);
 }
-
-__device__ void chem_res(const RelaxParams &R, const Ph *h, int pm, double *x, double rm, double re, double *r) {
-    const int mm = 1 - pm;
-    const double s1 = x[mm], s2 = x[mm] * x[mm + 2], s3 = x[mm] * x[mm + 2] * x[mm + 4];
-    x[pm] = 1 - s1;
-    x[pm + 2] = (rm - s2) / x[pm];
-    x[pm + 4] = (re - s3) / (x[pm] * x[pm + 2]);
-    double p[2], T[2];
+// the step h[q] of unknown q in the Jacobian
+__device__ __forceinline__ double chem_step(double x) { return fabs(x) < 1e-9 ? 1e-10 : 1.e-5 * x; }
+// points from <= q < to: 0 the base point (residuals), 1 .. 3 a, r, e stepped forward (Jacobian columns)
+__device__ __forceinline__ void chem_system(const RelaxParams &R, bool m1, double a, double r, double e, double rm, double re,
+                                            int from, int to, ChemSystem &S) {
+#pragma unroll 1
+    for (int q = from; q < to; q++) {
+        const double aq = q == 1 ? a + chem_step(a) : a;
+        const double rq = q == 2 ? r + chem_step(r) : r;
+        const double eq = q == 3 ? e + chem_step(e) : e;
+        const double ap = 1 - aq, part = rm - aq * rq;
+        const double rp = part / ap, ep = (re - aq * rq * eq) / part;
+        const double x0 = m1 ? rp : rq, x1 = m1 ? rq : rp;
+        double p[2], T[2];
+        p[0] = p_of(R, 0, x0, m1 ? ep : eq);
+        p[1] = p_of(R, 1, x1, m1 ? eq : ep);
+        T[0] = (p[0] + R.pinf[0]) / (R.cvgm1[0] * x0);
+        T[1] = (p[1] + R.pinf[1]) / (R.cvgm1[1] * x1);
+        ChemLog l;
+        const double d0 = (T[0] - S.T[0]) * S.iT[0], d1 = (T[1] - S.T[1]) * S.iT[1];
+        const double d2 = (p[0] - S.p[0]) * S.iP[0], d3 = (p[1] - S.p[1]) * S.iP[1];
+        if (q && fabs(d0) < kSmallLog && fabs(d1) < kSmallLog && fabs(d2) < kSmallLog && fabs(d3) < kSmallLog) {
+            l.lT[0] = S.log.lT[0] + log10_1p(d0);
+            l.lT[1] = S.log.lT[1] + log10_1p(d1);
+            l.lP[0] = S.log.lP[0] + log10_1p(d2);
+            l.lP[1] = S.log.lP[1] + log10_1p(d3);
+        } else {
+            l.lT[0] = log10(T[0]);
+            l.lT[1] = log10(T[1]);
+            l.lP[0] = log10(p[0] + R.pinf[0]);
+            l.lP[1] = log10(p[1] + R.pinf[1]);
+        }
+        l.lG = R.pinf[1] == 0.0 ? l.lP[1] : log10(p[1]);
+        const double g = chem_gibbs_diff(R, T, l);
+        if (q == 0) {
+            S.res[0] = p[0] - p[1];
+            S.res[1] = T[0] - T[1];
+            S.res[2] = g;
+            S.ap = ap;
+            S.rp = rp;
+            S.log = l;
 #pragma unroll
-    for (int m = 0; m < 2; m++) {
-        p[m] = p_of(h[m], x[m + 2], x[m + 4]);
-        T[m] = t_of(h[m], x[m + 2], x[m + 4]);
-    }
-    r[0] = p[0] - p[1];
-    r[1] = T[0] - T[1];
-    r[2] = gibbs_of(R, 0, p[0], T[0]) - gibbs_of(R, 1, p[1], T[1]);
-}
-
-__device__ void chem_check(const RelaxParams &R, double xOld, double *x, double dx, int i, float urf, int *ab, double rho) {
-    if (i == 0 || i == 1) {
-        if (x[i] < 0) { while (x[i] < R.chemLimit && urf > 0.0005f) { urf = urf / 2; x[i] = xOld - urf * dx; } }
-        if (x[i] > 1) { while (x[i] > 1.0 - R.chemLimit && urf > 0.0005f) { urf = urf / 2; x[i] = xOld - urf * dx; } }
-        if (x[i] < 0) *ab = 1;
-        if (x[i] > 1) *ab = 1;
-    } else if (i == 2 || i == 3) {
-        double ar = x[i - 2] * x[i];
-        if (x[i] < 0) { while (x[i] < 0 && urf > 0.0005f) { urf = urf / 2; x[i] = xOld - urf * dx; } }
-        if (ar > rho) { while (ar > rho && urf > 0.0005f) { urf = urf / 2; x[i] = xOld - urf * dx; ar = x[i - 2] * x[i]; } }
-        if (x[i] < 0) *ab = 1;
-        if (ar > rho) *ab = 1;
+            for (int m = 0; m < 2; m++) {
+                S.p[m] = p[m];
+                S.T[m] = T[m];
+                S.iT[m] = 1.0 / T[m];
+                S.iP[m] = 1.0 / (p[m] + R.pinf[m]);
+            }
+        } else {
+            const double ih = 1.0 / chem_step(q == 1 ? a : (q == 2 ? r : e));
+            const double c0 = ((p[0] - p[1]) - S.res[0]) * ih, c1 = ((T[0] - T[1]) - S.res[1]) * ih, c2 = (g - S.res[2]) * ih;
+            if (q == 1) { S.jac[0][0] = c0; S.jac[1][0] = c1; S.jac[2][0] = c2; }
+            if (q == 2) { S.jac[0][1] = c0; S.jac[1][1] = c1; S.jac[2][1] = c2; }
+            if (q == 3) { S.jac[0][2] = c0; S.jac[1][2] = c1; S.jac[2][2] = c2; }
+        }
     }
 }
 
-__device__ int chem_cell(const RelaxParams &R, const Ph *h, double *U, int *iters) {
-    double x[6], ax[6];
-    x[0] = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
-    x[1] = 1 - x[0];
-    x[2] = U[1] / x[0];
-    x[3] = U[2] / x[1];
-    x[4] = U[6] / (x[0] * x[2]);
-    x[5] = U[7] / (x[1] * x[3]);
-#pragma unroll
-    for (int i = 0; i < 6; i++) ax[i] = x[i];
-    const double rm = x[0] * x[2] + x[1] * x[3];
-    const double u = U[3] / rm, v = U[4] / rm, w = U[5] / rm;
-    const double re = U[8] - 0.5 * rm * (u * u + v * v + w * w);
-    const int pm = (x[1] > x[0]) ? 1 : 0;
-    const int mm = 1 - pm;
+// dx = jac^-1 res by cofactors; the determinant
+__device__ __forceinline__ double chem_direction(const ChemSystem &S, double *dx) {
+    const double(*j)[3] = S.jac;
+    const double c00 = j[1][1] * j[2][2] - j[1][2] * j[2][1];
+    const double c01 = j[1][0] * j[2][2] - j[1][2] * j[2][0];
+    const double c02 = j[1][0] * j[2][1] - j[1][1] * j[2][0];
+    const double det = j[0][0] * c00 - j[0][1] * c01 + j[0][2] * c02;
+    const double id = 1.0 / det;
+    dx[0] = id * (c00 * S.res[0] - (j[0][1] * j[2][2] - j[0][2] * j[2][1]) * S.res[1] +
+                  (j[0][1] * j[1][2] - j[0][2] * j[1][1]) * S.res[2]);
+    dx[1] = id * (-c01 * S.res[0] + (j[0][0] * j[2][2] - j[0][2] * j[2][0]) * S.res[1] -
+                  (j[0][0] * j[1][2] - j[0][2] * j[1][0]) * S.res[2]);
+    dx[2] = id * (c02 * S.res[0] - (j[0][0] * j[2][1] - j[0][1] * j[2][0]) * S.res[1] +
+                  (j[0][0] * j[1][1] - j[0][1] * j[1][0]) * S.res[2]);
+    return det;
+}
+
+// relaxed state from the minor phase's (a, r, e): the primary phase closes mass and energy
+__device__ __forceinline__ void chem_store(const RelaxParams &R, bool m1, double a, double r, double e, double rm, double re,
+                                           double *U) {
+    const double part = rm - a * r;
+    const double ap = 1 - a, rp = part / ap, ep = (re - a * r * e) / part;
+    const double x0 = m1 ? ap : a, r0 = m1 ? rp : r, r1 = m1 ? r : rp, e0 = m1 ? ep : e, e1 = m1 ? e : ep;
+    const double x1 = m1 ? a : ap;
+    U[0] = fmin(fmax(R.avfMin / 100, x0), 1 - R.avfMin / 100);
+    U[1] = x0 * r0;
+    U[2] = x1 * r1;
+    U[6] = x0 * r0 * e0;
+    U[7] = x1 * r1 * e1;
+    U[9] = x1 * r1;
+}
+
+// A step that left the unknown's range is halved until it is back (DP/chemRlx.cu:132-170): volume
+// fractions in [0, 1], partial densities in [0, rm].  1 where it stays outside.
+__device__ int chem_limit_fraction(const RelaxParams &R, double old, double &x, double dx) {
+    float urf = (float)R.chemUrf;
+    if (x < 0) { while (x < R.chemLimit && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; } }
+    if (x > 1) { while (x > 1.0 - R.chemLimit && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; } }
+    return x < 0 || x > 1;
+}
+__device__ int chem_limit_density(const RelaxParams &R, double a, double old, double &x, double dx, double rm) {
+    float urf = (float)R.chemUrf;
+    double ar = a * x;
+    if (x < 0) { while (x < 0 && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; } }
+    if (ar > rm) { while (ar > rm && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; ar = a * x; } }
+    return x < 0 || ar > rm;
+}
+
+// Chemical equilibrium (DP/chemRlx.cu:4-267): damped Newton from the cell's state
+__device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
+    double a, r, e, rm, re;
+    bool m1;
+    {
+        const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100), a1 = 1 - a0;
+        const double r0 = U[1] / a0, r1 = U[2] / a1;
+        const double e0 = U[6] / (a0 * r0), e1 = U[7] / (a1 * r1);
+        rm = a0 * r0 + a1 * r1;
+        const double u = U[3] / rm, v = U[4] / rm, w = U[5] / rm;
+        re = U[8] - 0.5 * rm * (u * u + v * v + w * w);
+        m1 = !(a1 > a0);
+        a = m1 ? a1 : a0;
+        r = m1 ? r1 : r0;
+        e = m1 ? e1 : e0;
+    }
+    double ba = a, br = r, be = e;   // best iterate
     float minRes = 1e9f;
-    int abortFlag = 0, aborted = 0;
+    int aborted = 0;
     for (int itr = 1;; itr++) {
         *iters = itr;
-        double res[3], rdf[3][3], e[3];
-        chem_res(R, h, pm, x, rm, re, res);
-        const int js[3] = {mm, mm + 2, mm + 4};
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const int j = js[q];
-            e[q] = fabs(x[j]) < 1e-9 ? 1e-10 : 1.e-5 * x[j];
-            x[j] += e[q];
-            double rr[3];
-            chem_res(R, h, pm, x, rm, re, rr);
-            rdf[0][q] = rr[0]; rdf[1][q] = rr[1]; rdf[2][q] = rr[2];
-            x[j] -= e[q];
-        }
-        double j_[3][3];
+        ChemSystem S;
+        chem_system(R, m1, a, r, e, rm, re, 0, 4, S);
+        double dx[3];
+        const double det = chem_direction(S, dx);
+        int ab = det == 0;
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-                j_[i][j] = (rdf[i][j] - res[i]) / e[j];
-                if (isnan(j_[i][j])) abortFlag = 1;
-            }
-        const double det = j_[0][0] * (j_[1][1] * j_[2][2] - j_[1][2] * j_[2][1]) -
-                           j_[0][1] * (j_[1][0] * j_[2][2] - j_[1][2] * j_[2][0]) +
-                           j_[0][2] * (j_[1][0] * j_[2][1] - j_[1][1] * j_[2][0]);
-        if (det == 0) abortFlag = 1;
-        const double id = 1.0 / det;
-        double inv[3][3];
-        inv[0][0] = id * (j_[1][1] * j_[2][2] - j_[1][2] * j_[2][1]);
-        inv[0][1] = -id * (j_[0][1] * j_[2][2] - j_[0][2] * j_[2][1]);
-        inv[0][2] = id * (j_[0][1] * j_[1][2] - j_[0][2] * j_[1][1]);
-        inv[1][0] = -id * (j_[1][0] * j_[2][2] - j_[1][2] * j_[2][0]);
-        inv[1][1] = id * (j_[0][0] * j_[2][2] - j_[0][2] * j_[2][0]);
-        inv[1][2] = -id * (j_[0][0] * j_[1][2] - j_[0][2] * j_[1][0]);
-        inv[2][0] = id * (j_[1][0] * j_[2][1] - j_[1][1] * j_[2][0]);
-        inv[2][1] = -id * (j_[0][0] * j_[2][1] - j_[0][1] * j_[2][0]);
-        inv[2][2] = id * (j_[0][0] * j_[1][1] - j_[0][1] * j_[1][0]);
-        if (abortFlag == 0 && x[0] > 0.0 && x[0] < 1.0 && x[1] > 0.0 && x[1] < 1.0 && x[2] > 0.0 && x[3] > 0.0) {
-            const float chk = sqrt(res[0] * res[0] + res[1] * res[1] + res[2] * res[2]);
+            for (int j = 0; j < 3; j++) ab |= isnan(S.jac[i][j]);
+        if (!ab && a > 0.0 && a < 1.0 && S.ap > 0.0 && S.ap < 1.0 && r > 0.0 && S.rp > 0.0) {
+            const float chk = sqrt(S.res[0] * S.res[0] + S.res[1] * S.res[1] + S.res[2] * S.res[2]);
             if (chk < minRes) {
                 minRes = chk;
-#pragma unroll
-                for (int i = 0; i < 6; i++) ax[i] = x[i];
+                ba = a;
+                br = r;
+                be = e;
             }
         }
-        int abLocal = abortFlag;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const int i = js[q];
-            const double dx = inv[q][0] * res[0] + inv[q][1] * res[1] + inv[q][2] * res[2];
-            x[i] = x[i] - R.chemUrf * dx;
-            chem_check(R, x[i] + R.chemUrf * dx, x, dx, i, (float)R.chemUrf, &abLocal, rm);
-        }
-        const bool conv = !(fabs(res[0]) > 1.e-1) && !(fabs(res[1]) > 1.e-1) && !(fabs(res[2]) > 1.e-1);
-        if (abLocal == 1 || itr > R.chemItrMax) {
-#pragma unroll
-            for (int i = 0; i < 6; i++) x[i] = ax[i];
+        const double oa = a, orr = r;
+        a = a - R.chemUrf * dx[0];
+        ab |= chem_limit_fraction(R, oa, a, dx[0]);
+        r = r - R.chemUrf * dx[1];
+        ab |= chem_limit_density(R, a, orr, r, dx[1], rm);
+        e = e - R.chemUrf * dx[2];
+        if (ab || itr > R.chemItrMax) {
+            a = ba;
+            r = br;
+            e = be;
             aborted = 1;
             break;
         }
-        if (conv) break;
+        if (!(fabs(S.res[0]) > 1.e-1) && !(fabs(S.res[1]) > 1.e-1) && !(fabs(S.res[2]) > 1.e-1)) break;
     }
-    const double s1 = x[mm], s2 = x[mm] * x[mm + 2], s3 = x[mm] * x[mm + 2] * x[mm + 4];
-    x[pm] = 1 - s1;
-    x[pm + 2] = (rm - s2) / x[pm];
-    x[pm + 4] = (re - s3) / (x[pm] * x[pm + 2]);
-    U[0] = fmin(fmax(R.avfMin / 100, x[0]), 1 - R.avfMin / 100);
-    U[1] = x[0] * x[2];
-    U[2] = x[1] * x[3];
-    U[6] = x[0] * x[2] * x[4];
-    U[7] = x[1] * x[3] * x[5];
-    U[9] = x[1] * x[3];
+    chem_store(R, m1, a, r, e, rm, re, U);
     return aborted;
 }
 
@@ -280,89 +347,56 @@ __device__ __forceinline__ void chem_mixture(const RelaxParams &R, const double 
     *ag = a1 * r1;
 }
 
-// Full-step Newton from the surrogate's equilibrium (p, T, alpha) on the residuals of chem_res.
+// Full-step Newton from the surrogate's equilibrium (p, T, alpha) on the residuals of chem_system.
 // Returns 1 and writes U when every relative residual is within relTol.
-__device__ int chem_polish(const RelaxParams &R, const Ph *h, double *U, const float *y, double rm, double re,
-                           double relTol, int maxIt, int *iters) {
+__device__ int chem_polish(const RelaxParams &R, double *U, const float *y, double rm, double re, double relTol, int maxIt,
+                           int *iters) {
     const double p = y[0], T = y[1];
-    if (!(T > 0) || !(p > -h[0].pinf) || !(p > -h[1].pinf)) return 0;
-    double x[6];
-    const double rL = (p + h[0].pinf) / ((h[0].cp / h[0].g) * (h[0].g - 1) * T);
-    const double rG = (p + h[1].pinf) / ((h[1].cp / h[1].g) * (h[1].g - 1) * T);
-    double a = (rm - rG) / (rL - rG);   // mass balance at (p, T)
-    if (!(a > 0 && a < 1)) a = y[2];
-    if (!(a > 0 && a < 1)) return 0;
-    x[0] = a;
-    x[1] = 1 - a;
-    x[2] = rL;
-    x[3] = rG;
-    x[4] = (p + h[0].g * h[0].pinf) / ((h[0].g - 1) * rL) + h[0].eta;
-    x[5] = (p + h[1].g * h[1].pinf) / ((h[1].g - 1) * rG) + h[1].eta;
-    const int pm = (x[1] > x[0]) ? 1 : 0, mm = 1 - pm;
-    const double sp = fmax(fabs(p), 1.0), sT = T, sg = h[0].cp * T;
+    if (!(T > 0) || !(p > -R.pinf[0]) || !(p > -R.pinf[1])) return 0;
+    const double rL = (p + R.pinf[0]) / (R.cvgm1[0] * T);
+    const double rG = (p + R.pinf[1]) / (R.cvgm1[1] * T);
+    double al = (rm - rG) / (rL - rG);   // mass balance at (p, T)
+    if (!(al > 0 && al < 1)) al = y[2];
+    if (!(al > 0 && al < 1)) return 0;
+    const bool m1 = !(1 - al > al);
+    double a = m1 ? 1 - al : al, r = m1 ? rG : rL;
+    double e = m1 ? (p + R.gpinf[1]) / (R.gm1[1] * rG) + R.eta[1] : (p + R.gpinf[0]) / (R.gm1[0] * rL) + R.eta[0];
+    const double sp = fmax(fabs(p), 1.0), sT = T, sg = R.cp[0] * T;
     int ok = 0;
     for (int itr = 0; itr <= maxIt; itr++) {
-        double res[3];
-        chem_res(R, h, pm, x, rm, re, res);
-        if (!(x[0] > 0 && x[0] < 1 && x[2] > 0 && x[3] > 0)) break;
-        if (fabs(res[0]) <= relTol * sp && fabs(res[1]) <= relTol * sT && fabs(res[2]) <= relTol * sg) {
+        ChemSystem S;
+        chem_system(R, m1, a, r, e, rm, re, 0, 1, S);
+        if (!(a > 0 && a < 1 && r > 0 && S.rp > 0)) break;
+        if (fabs(S.res[0]) <= relTol * sp && fabs(S.res[1]) <= relTol * sT && fabs(S.res[2]) <= relTol * sg) {
             ok = 1;
             break;
         }
         if (itr == maxIt) break;
         *iters = itr + 1;
-        const int js[3] = {mm, mm + 2, mm + 4};
-        double jac[3][3], e[3];
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const int j = js[q];
-            e[q] = fabs(x[j]) < 1e-9 ? 1e-10 : 1.e-5 * x[j];
-            x[j] += e[q];
-            double rr[3];
-            chem_res(R, h, pm, x, rm, re, rr);
-            x[j] -= e[q];
-#pragma unroll
-            for (int i = 0; i < 3; i++) jac[i][q] = (rr[i] - res[i]) / e[q];
-        }
-        const double det = jac[0][0] * (jac[1][1] * jac[2][2] - jac[1][2] * jac[2][1]) -
-                           jac[0][1] * (jac[1][0] * jac[2][2] - jac[1][2] * jac[2][0]) +
-                           jac[0][2] * (jac[1][0] * jac[2][1] - jac[1][1] * jac[2][0]);
+        chem_system(R, m1, a, r, e, rm, re, 1, 4, S);
+        double dx[3];
+        const double det = chem_direction(S, dx);
         if (!(fabs(det) > 0) || !isfinite(det)) break;
-        const double id = 1.0 / det;
-        double inv[3][3];
-        inv[0][0] = id * (jac[1][1] * jac[2][2] - jac[1][2] * jac[2][1]);
-        inv[0][1] = -id * (jac[0][1] * jac[2][2] - jac[0][2] * jac[2][1]);
-        inv[0][2] = id * (jac[0][1] * jac[1][2] - jac[0][2] * jac[1][1]);
-        inv[1][0] = -id * (jac[1][0] * jac[2][2] - jac[1][2] * jac[2][0]);
-        inv[1][1] = id * (jac[0][0] * jac[2][2] - jac[0][2] * jac[2][0]);
-        inv[1][2] = -id * (jac[0][0] * jac[1][2] - jac[0][2] * jac[1][0]);
-        inv[2][0] = id * (jac[1][0] * jac[2][1] - jac[1][1] * jac[2][0]);
-        inv[2][1] = -id * (jac[0][0] * jac[2][1] - jac[0][1] * jac[2][0]);
-        inv[2][2] = id * (jac[0][0] * jac[1][1] - jac[0][1] * jac[1][0]);
-#pragma unroll
-        for (int q = 0; q < 3; q++) x[js[q]] -= inv[q][0] * res[0] + inv[q][1] * res[1] + inv[q][2] * res[2];
+        a -= dx[0];
+        r -= dx[1];
+        e -= dx[2];
     }
     if (!ok) return 0;
-    U[0] = fmin(fmax(R.avfMin / 100, x[0]), 1 - R.avfMin / 100);
-    U[1] = x[0] * x[2];
-    U[2] = x[1] * x[3];
-    U[6] = x[0] * x[2] * x[4];
-    U[7] = x[1] * x[3] * x[5];
-    U[9] = x[1] * x[3];
+    chem_store(R, m1, a, r, e, rm, re, U);
     return 1;
 }
 
 // partitionRelaxation (DP/relaxation.cu:4-75): the cell needs the chemical (Gibbs) solve when its
 // liquid temperature is above the saturation temperature at its liquid pressure and its
 // volume fraction above chemLimit
-__device__ __forceinline__ int needs_chem(const RelaxParams &R, const Ph *h, const double *u) {
+__device__ __forceinline__ int needs_chem(const RelaxParams &R, const double *u) {
     const double avf = fmin(fmax(R.avfMin / 100, u[0]), 1 - R.avfMin / 100);
+    if (!(avf > R.chemLimit)) return 0;   // whatever its saturation temperature
     const double rho = u[1] / avf;
     const double enr = u[6] / (avf * rho);
-    const double tl = t_of(h[0], rho, enr);
-    const double pl = p_of(h[0], rho, enr);
-    const double ts = sat_temp(R, pl, tl, R.satTempUrf);
-    return (tl > ts && avf > R.chemLimit);
+    const double tl = t_of(R, 0, rho, enr);
+    const double pl = p_of(R, 0, rho, enr);
+    return tl > sat_temp(R, pl, tl, R.satTempUrf);
 }
 
 }  // namespace
@@ -377,12 +411,11 @@ __global__ void k_relax_partition(int n, const double *__restrict__ U, const Rel
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     int chem = 0;
     if (c < n) {
-        const Ph h[2] = {{R.gam[0], R.pinf[0], R.cp[0], R.eta[0]}, {R.gam[1], R.pinf[1], R.cp[1], R.eta[1]}};
         double u[NV];
         u[0] = U[c];
         u[1] = U[(size_t)n + c];
         u[6] = U[(size_t)6 * n + c];
-        chem = needs_chem(R, h, u);
+        chem = needs_chem(R, u);
         isChem[c] = (uint8_t)chem;
     }
     const int cnt = __syncthreads_count(chem);
@@ -495,7 +528,6 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
                                                const SurrogateDev S, const int32_t *order, const int32_t *nChem,
                                                const float4 *pred, int32_t *hullOk) {
     const int m = *nChem;
-    const Ph h[2] = {{R.gam[0], R.pinf[0], R.cp[0], R.eta[0]}, {R.gam[1], R.pinf[1], R.cp[1], R.eta[1]}};
     // base is the same for every thread of the block: the warp collectives below see full warps
     for (int base = blockIdx.x * blockDim.x; base < m; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
@@ -509,7 +541,7 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
             chem_mixture(R, u, &rm, &re, &ag);
             const float4 p4 = pred[i];
             const float pr[4] = {p4.x, p4.y, p4.z, p4.w};
-            used = chem_polish(R, h, u, pr, rm, re, S.relTol, S.polishIters, &pits);
+            used = chem_polish(R, u, pr, rm, re, S.relTol, S.polishIters, &pits);
             if (used) {
                 U[(size_t)0 * n + c] = u[0];
                 U[(size_t)1 * n + c] = u[1];
@@ -545,7 +577,6 @@ __global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINB
     const bool act = i < n;
     const int c = (kOrd && act) ? order[i] : i;
     int chem = 0, ab = 0, its = 0, used = 0, pits = 0;
-    const Ph h[2] = {{R.gam[0], R.pinf[0], R.cp[0], R.eta[0]}, {R.gam[1], R.pinf[1], R.cp[1], R.eta[1]}};
     double u[NV];
     double rm = 0, re = 0, ag = 0;
     if (act) {
@@ -564,10 +595,10 @@ __global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINB
         if (kPolish && chem && hullOk[i] != 0) {
             const float4 p4 = pred[i];
             const float pr[4] = {p4.x, p4.y, p4.z, p4.w};
-            used = chem_polish(R, h, u, pr, rm, re, S.relTol, S.polishIters, &pits);
+            used = chem_polish(R, u, pr, rm, re, S.relTol, S.polishIters, &pits);
         }
         if (!used) {
-            ab = (kOrd && chem) ? chem_cell(R, h, u, &its) : therm_cell(R, h, u, &its);
+            ab = (kOrd && chem) ? chem_cell(R, u, &its) : therm_cell(R, u, &its);
         }
         if (kLog && chem && !used && !ab) {
             // training sample: (rho, e, Y) before the solve -> (p, T, alpha, Y_eq) after it
@@ -579,8 +610,8 @@ __global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINB
                 x[0] = (float)rm;
                 x[1] = (float)(re / rm);
                 x[2] = (float)(ag / rm);
-                y[0] = (float)p_of(h[0], rL, eL);
-                y[1] = (float)t_of(h[0], rL, eL);
+                y[0] = (float)p_of(R, 0, rL, eL);
+                y[1] = (float)t_of(R, 0, rL, eL);
                 y[2] = (float)a0;
                 y[3] = (float)(u[9] / rm);
             }

@@ -359,6 +359,20 @@ struct SolverT : public fg_solver {
             R.cp[k] = cs.Cp[k];
             R.eta[k] = cs.eta[k];
             R.satConst[k] = cs.satConst[k];
+            R.gm1[k] = g - 1;
+            R.gpinf[k] = g * cs.pInf[k];
+            R.gm1eta[k] = (g - 1) * cs.eta[k];
+            R.cv[k] = cs.Cp[k] / g;
+            R.cvgm1[k] = (cs.Cp[k] / g) * (g - 1);
+        }
+        {
+            // saturation line (DP/relaxation.cu:4-38)
+            const double q = R.cp[1] - R.cv[1];
+            R.satA = R.cp[0] - R.cp[1];
+            R.satQ = 1.0 / q;
+            R.satB = (R.eta[0] - R.eta[1]) / q;
+            R.satC = (R.cp[1] - R.cp[0]) / q;
+            R.satD = (R.cp[0] - R.cv[0]) / q;
         }
         D.avfLo = cs.avfMin / 100;
         D.avfHi = 1.0 - cs.avfMin / 100;
