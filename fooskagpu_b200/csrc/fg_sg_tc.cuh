@@ -124,11 +124,6 @@ __device__ __forceinline__ bool tc_layer(unsigned char *sm, uint32_t tmem, int w
     return ok;
 }
 
-// byte offset of (row, k) as above, for host-side packing
-inline uint32_t tc_smem_off_host(int row, int k, int rows) {
-    return (uint32_t)((k >> 4) * rows * 32 + (row >> 3) * 256 + ((k >> 3) & 1) * 128 + (row & 7) * 16 + (k & 7) * 2);
-}
-
 // Evaluate the network for the samples of `in` (tiles of 128, persistent CTAs): out[i] = raw
 // outputs (p, T, alpha, Y_eq), hull[i] = inside the training hull.  `wpack` holds the four
 // layers' weights in the canonical layout (TC_WBYTES bytes); *err = 1 if an MMA completion wait

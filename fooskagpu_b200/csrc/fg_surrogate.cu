@@ -54,112 +54,298 @@ struct Buf {
                                  std::string(#expr) + ": " + cudaGetErrorString(e_));                 \
     } while (0)
 
-constexpr int kChunks = 64;   // sample chunks of the weight-gradient reduction
+// ---- one training pass over a batch: forward, loss, backward and weight gradients in one kernel,
+// then a reduction over its blocks with the Adam step.
+//
+// A block of 256 threads takes tiles of kTrainS samples (grid-stride, kTrainS small enough that a
+// 4096-sample batch fills the SMs), keeps the parameters and the tile's activations in shared
+// memory, and accumulates its share of every weight gradient in registers over its tiles; the
+// block's sums go to part[block][SG_NPARAM] once, at the end.  Bound by FP32 multiply-adds from
+// shared memory (26 k per sample): a thread computes 2 samples x 4 outputs of a layer (one 16-byte
+// read of a weight row feeds 8 multiply-adds), 4 x 4 of a weight gradient.  Rows have a pitch of 68
+// values, so that 8 lanes reading 16 bytes of 8 consecutive rows hit distinct banks.
+// Summation order: a block's samples in order, then the blocks in a fixed order, so training is
+// deterministic for a given batch size.
+// Measured (B200, batch 4096): 17.9 us, and 3 us for the reduction, against 230 us for the 15 launches of
+// one layer or one reduction each that it replaced; an epoch of 16 batches 4.44 -> 0.70 ms.
+constexpr int kTrainS = 32, kTrainThreads = 256, kTrainPitch = SG_H + 4;
+constexpr int kTrainMaxBlocks = 296;   // 2 resident blocks on each of 148 SMs
+constexpr int kTrainRows = kTrainS * kTrainPitch;
+// shared memory (values): W2, W3 with padded rows, W1, W4, biases; per layer the tile's activations
+// and the derivative of its GELU (then its dZ); inputs, targets, output gradients
+constexpr int TS_W2 = 0, TS_W3 = TS_W2 + SG_H * kTrainPitch, TS_W1 = TS_W3 + SG_H * kTrainPitch,
+              TS_W4 = TS_W1 + SG_IN * SG_H, TS_B = TS_W4 + SG_H * SG_OUT, TS_A = TS_B + 3 * SG_H + SG_OUT,
+              TS_D = TS_A + 3 * kTrainRows, TS_X = TS_D + 3 * kTrainRows, TS_Y = TS_X + kTrainS * 4,
+              TS_G = TS_Y + kTrainS * SG_OUT, TS_RED = TS_G + kTrainS * SG_OUT, TS_END = TS_RED + 8;
+static_assert(TS_A % 4 == 0 && TS_W4 % 4 == 0 && TS_X % 4 == 0, "16-byte aligned rows");
 
-// GELU (tanh form) and its derivative in training: with u = c (z + a z^3), th = tanh(u),
+// GELU (tanh form) and its derivative: with u = c (z + a z^3), th = tanh(u),
 //   gelu = z / 2 (1 + th),  gelu' = (1 + th) / 2 + z / 2 (1 - th^2) c (1 + 3 a z^2)
-__device__ __forceinline__ float gelu_f(float z) {
-    return 0.5f * z * (1.0f + tanhf(SG_GELU_C * fmaf(SG_GELU_A * z, z * z, z)));
-}
-__device__ __forceinline__ float gelu_d(float z) {
+__device__ __forceinline__ float gelu_fd(float z, float &d) {
     const float th = tanhf(SG_GELU_C * fmaf(SG_GELU_A * z, z * z, z));
-    return 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * SG_GELU_C * fmaf(3.0f * SG_GELU_A * z, z, 1.0f);
+    d = 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * SG_GELU_C * fmaf(3.0f * SG_GELU_A * z, z, 1.0f);
+    return 0.5f * z * (1.0f + th);
 }
-
-// rows of X and Y selected by perm[start .. start+B)
-__global__ void k_sg_gather(const int32_t *perm, int start, int B, const float *X, const float *Y, float *bx,
-                            float *by) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B) return;
-    const int s = perm[start + i];
-#pragma unroll
-    for (int k = 0; k < SG_IN; k++) bx[(size_t)i * SG_IN + k] = X[(size_t)s * SG_IN + k];
-#pragma unroll
-    for (int k = 0; k < SG_OUT; k++) by[(size_t)i * SG_OUT + k] = Y[(size_t)s * SG_OUT + k];
+__device__ __forceinline__ void fma4(float4 &c, float a, const float4 &w) {
+    c.x = fmaf(a, w.x, c.x);
+    c.y = fmaf(a, w.y, c.y);
+    c.z = fmaf(a, w.z, c.z);
+    c.w = fmaf(a, w.w, c.w);
 }
-
-// Z = X W + b (X: B x K, W: K x N row-major), A = gelu(Z) (act) or Z
-__global__ void k_dense_fwd(const float *X, int K, const float *W, const float *b, int N, int B, float *Z, float *A,
-                            int act) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * N) return;
-    const int r = i / N, n = i - r * N;
-    float z = b[n];
-    for (int k = 0; k < K; k++) z = fmaf(X[(size_t)r * K + k], W[k * N + n], z);
-    if (Z) Z[i] = z;
-    A[i] = act ? gelu_f(z) : z;
+__device__ __forceinline__ float dot4(float c, const float4 &a, const float4 &w) {
+    return fmaf(a.w, w.w, fmaf(a.z, w.z, fmaf(a.y, w.y, fmaf(a.x, w.x, c))));
 }
-
-// dY = 2 (Y - T) / (B * 4); per-block partial sums of the squared error
-__global__ void k_sg_loss(const float *Yp, const float *Tt, int cnt, float scale, float *dY, float *part) {
-    __shared__ float sh[256];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float e = 0.f;
-    if (i < cnt) {
-        const float d = Yp[i] - Tt[i];
-        dY[i] = 2.f * d * scale;
-        e = d * d;
+// store the GELU of a thread's 4 pre-activations of a sample and its derivative
+__device__ __forceinline__ void train_act(float *A, float *D, int s, int n, const float4 &z) {
+    float4 a, d;
+    a.x = gelu_fd(z.x, d.x);
+    a.y = gelu_fd(z.y, d.y);
+    a.z = gelu_fd(z.z, d.z);
+    a.w = gelu_fd(z.w, d.w);
+    *reinterpret_cast<float4 *>(A + s * kTrainPitch + n) = a;
+    *reinterpret_cast<float4 *>(D + s * kTrainPitch + n) = d;
+}
+// hidden layer: A = gelu(P W + b) for the thread's samples s0, s0 + 1 and outputs n .. n + 3
+__device__ __forceinline__ void train_fwd(const float *W, const float *b, const float *P, float *A, float *D, int s0, int n) {
+    float4 z0 = *reinterpret_cast<const float4 *>(b + n), z1 = z0;
+#pragma unroll 4
+    for (int k = 0; k < SG_H; k += 4) {
+        const float4 p0 = *reinterpret_cast<const float4 *>(P + s0 * kTrainPitch + k);
+        const float4 p1 = *reinterpret_cast<const float4 *>(P + (s0 + 1) * kTrainPitch + k);
+        const float *w = W + k * kTrainPitch + n;
+        float4 r = *reinterpret_cast<const float4 *>(w);
+        fma4(z0, p0.x, r);
+        fma4(z1, p1.x, r);
+        r = *reinterpret_cast<const float4 *>(w + kTrainPitch);
+        fma4(z0, p0.y, r);
+        fma4(z1, p1.y, r);
+        r = *reinterpret_cast<const float4 *>(w + 2 * kTrainPitch);
+        fma4(z0, p0.z, r);
+        fma4(z1, p1.z, r);
+        r = *reinterpret_cast<const float4 *>(w + 3 * kTrainPitch);
+        fma4(z0, p0.w, r);
+        fma4(z1, p1.w, r);
     }
-    sh[threadIdx.x] = e;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+    train_act(A, D, s0, n, z0);
+    train_act(A, D, s0 + 1, n, z1);
+}
+// backward data: D (derivative of the layer below, becomes its dZ) *= dZ W^T, for the thread's samples
+// s0, s0 + 1 and inputs kk, kk + 16, kk + 32, kk + 48
+__device__ __forceinline__ void train_bwd(const float *W, const float *dZ, float *D, int s0, int kk) {
+    float c[2][4] = {};
+#pragma unroll 4
+    for (int n = 0; n < SG_H; n += 4) {
+        const float4 d0 = *reinterpret_cast<const float4 *>(dZ + s0 * kTrainPitch + n);
+        const float4 d1 = *reinterpret_cast<const float4 *>(dZ + (s0 + 1) * kTrainPitch + n);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float4 w = *reinterpret_cast<const float4 *>(W + (kk + 16 * j) * kTrainPitch + n);
+            c[0][j] = dot4(c[0][j], d0, w);
+            c[1][j] = dot4(c[1][j], d1, w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) D[(s0 + i) * kTrainPitch + kk + 16 * j] *= c[i][j];
+}
+// weight gradient of a hidden layer: g[i] += sum over the tile's samples of A[k0 + i] dZ[n .. n + 3];
+// gb += the sums of dZ (the bias gradient, used by the threads of the first row group)
+__device__ __forceinline__ void train_wgrad(const float *A, const float *dZ, int k0, int n, float4 *g, float4 &gb) {
+#pragma unroll 4
+    for (int s = 0; s < kTrainS; s++) {
+        const float4 a = *reinterpret_cast<const float4 *>(A + s * kTrainPitch + k0);
+        const float4 d = *reinterpret_cast<const float4 *>(dZ + s * kTrainPitch + n);
+        fma4(g[0], a.x, d);
+        fma4(g[1], a.y, d);
+        fma4(g[2], a.z, d);
+        fma4(g[3], a.w, d);
+        if (k0 == 0) fma4(gb, 1.0f, d);
+    }
+}
+
+// X [.][3], Y [.][4]: the batch's samples are rows perm[0 .. B) (rows 0 .. B without perm); scale =
+// 1 / (4 B).  lossPart[block]: the block's sum of squared errors.
+__global__ void __launch_bounds__(kTrainThreads, 2) k_sg_train(const float *__restrict__ P, const float *__restrict__ X,
+                                                               const float *__restrict__ Y, const int32_t *__restrict__ perm,
+                                                               int B, float scale, float *__restrict__ part,
+                                                               float *__restrict__ lossPart) {
+    extern __shared__ __align__(16) float sm[];
+    const int t = threadIdx.x;
+    for (int q = t; q < SG_H * SG_H; q += kTrainThreads) {
+        const int o = (q / SG_H) * kTrainPitch + q % SG_H;
+        sm[TS_W2 + o] = P[SG_OFF_W2 + q];
+        sm[TS_W3 + o] = P[SG_OFF_W3 + q];
+    }
+    if (t < SG_IN * SG_H) sm[TS_W1 + t] = P[SG_OFF_W1 + t];
+    sm[TS_W4 + t] = P[SG_OFF_W4 + t];
+    if (t < SG_H) {
+        sm[TS_B + t] = P[SG_OFF_B1 + t];
+        sm[TS_B + SG_H + t] = P[SG_OFF_B2 + t];
+        sm[TS_B + 2 * SG_H + t] = P[SG_OFF_B3 + t];
+    }
+    if (t < SG_OUT) sm[TS_B + 3 * SG_H + t] = P[SG_OFF_B4 + t];
+    float *A1 = sm + TS_A, *A2 = A1 + kTrainRows, *A3 = A2 + kTrainRows;
+    float *D1 = sm + TS_D, *D2 = D1 + kTrainRows, *D3 = D2 + kTrainRows;
+    // the thread's 2 x 4 part of a layer (forward: outputs n ..; backward: inputs kk ..) and 4 x 4
+    // part of a weight gradient (rows k0 .., columns n ..)
+    const int kk = t & 15, n = 4 * kk, s0 = 2 * (t >> 4), k0 = 4 * (t >> 4);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g2[4] = {zero, zero, zero, zero}, g3[4] = {zero, zero, zero, zero}, b2 = zero, b3 = zero;
+    float g1 = 0.f, g4 = 0.f, b4 = 0.f, loss = 0.f;
+    for (int tile = blockIdx.x; tile * kTrainS < B; tile += gridDim.x) {
+        __syncthreads();   // the parameters are there, the previous tile is done
+        if (t < kTrainS * 4) {
+            const int r = tile * kTrainS + (t >> 2), c = t & 3;
+            const int row = r < B ? (perm ? perm[r] : r) : -1;
+            // inputs with a 1 for the bias gradient of the first layer; a missing sample adds nothing
+            sm[TS_X + t] = row >= 0 ? (c < SG_IN ? X[(size_t)row * SG_IN + c] : 1.0f) : 0.0f;
+            sm[TS_Y + t] = row >= 0 ? Y[(size_t)row * SG_OUT + c] : 0.0f;
+        }
         __syncthreads();
+        {
+            const float4 w0 = *reinterpret_cast<const float4 *>(sm + TS_W1 + n), bz = *reinterpret_cast<const float4 *>(sm + TS_B + n);
+            const float4 w1 = *reinterpret_cast<const float4 *>(sm + TS_W1 + SG_H + n);
+            const float4 w2 = *reinterpret_cast<const float4 *>(sm + TS_W1 + 2 * SG_H + n);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float4 x = *reinterpret_cast<const float4 *>(sm + TS_X + 4 * (s0 + i));
+                float4 z = bz;
+                fma4(z, x.x, w0);
+                fma4(z, x.y, w1);
+                fma4(z, x.z, w2);
+                train_act(A1, D1, s0 + i, n, z);
+            }
+        }
+        __syncthreads();
+        train_fwd(sm + TS_W2, sm + TS_B + SG_H, A1, A2, D2, s0, n);
+        __syncthreads();
+        train_fwd(sm + TS_W3, sm + TS_B + 2 * SG_H, A2, A3, D3, s0, n);
+        __syncthreads();
+        {
+            // output layer and loss: sample t / 8, output (t / 2) % 4, half of the inputs t % 2
+            const int s = t >> 3, o = (t >> 1) & 3, h = (t & 1) * (SG_H / 2);
+            float y = 0.f;
+#pragma unroll 8
+            for (int k = 0; k < SG_H / 2; k++) y = fmaf(A3[s * kTrainPitch + h + k], sm[TS_W4 + (h + k) * SG_OUT + o], y);
+            y += __shfl_xor_sync(0xffffffffu, y, 1);
+            if (!(t & 1)) {
+                const bool on = tile * kTrainS + s < B;
+                const float d = on ? y + sm[TS_B + 3 * SG_H + o] - sm[TS_Y + s * SG_OUT + o] : 0.0f;
+                sm[TS_G + s * SG_OUT + o] = 2.f * d * scale;
+                loss = fmaf(d, d, loss);
+            }
+        }
+        __syncthreads();
+        {
+            // gradients of the output layer (one weight per thread) and dZ of the third
+            const int k = t >> 2, o = t & 3;
+            float b = 0.f;
+#pragma unroll 8
+            for (int s = 0; s < kTrainS; s++) {
+                g4 = fmaf(A3[s * kTrainPitch + k], sm[TS_G + s * SG_OUT + o], g4);
+                b += sm[TS_G + s * SG_OUT + o];
+            }
+            b4 += b;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float4 d = *reinterpret_cast<const float4 *>(sm + TS_G + (s0 + i) * SG_OUT);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    D3[(s0 + i) * kTrainPitch + kk + 16 * j] *=
+                        dot4(0.f, d, *reinterpret_cast<const float4 *>(sm + TS_W4 + (kk + 16 * j) * SG_OUT));
+            }
+        }
+        __syncthreads();
+        train_bwd(sm + TS_W3, D3, D2, s0, kk);
+        train_wgrad(A2, D3, k0, n, g3, b3);
+        __syncthreads();
+        train_bwd(sm + TS_W2, D2, D1, s0, kk);
+        train_wgrad(A1, D2, k0, n, g2, b2);
+        __syncthreads();
+        {
+            // first layer: weight row t / 64 (row 3: the bias) and column t % 64
+            const int k = t >> 6, c = t & 63;
+#pragma unroll 8
+            for (int s = 0; s < kTrainS; s++) g1 = fmaf(sm[TS_X + 4 * s + k], D1[s * kTrainPitch + c], g1);
+        }
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// dX = (dZ W^T) * gelu'(Zprev)  (dZ: B x N, W: K x N, Zprev: B x K)
-__global__ void k_dense_bwd_data(const float *dZ, const float *W, int N, int K, const float *Zprev, int B,
-                                 float *dX) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * K) return;
-    const int r = i / K, k = i - r * K;
-    float s = 0.f;
-    for (int n = 0; n < N; n++) s = fmaf(dZ[(size_t)r * N + n], W[k * N + n], s);
-    dX[i] = s * gelu_d(Zprev[i]);
-}
-
-// partial weight / bias gradients over one chunk of samples:
-// part[chunk][k*N+n] = sum_r A[r][k] dZ[r][n],  part[chunk][K*N+n] = sum_r dZ[r][n]
-__global__ void k_dense_bwd_w(const float *A, const float *dZ, int B, int K, int N, int chunk, float *part) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nq = K * N + N;
-    if (q >= nq) return;
-    const int c = blockIdx.y;
-    const int r0 = c * chunk, r1 = min(B, r0 + chunk);
-    float s = 0.f;
-    if (q < K * N) {
-        const int k = q / N, n = q - k * N;
-        for (int r = r0; r < r1; r++) s = fmaf(A[(size_t)r * K + k], dZ[(size_t)r * N + n], s);
-    } else {
-        const int n = q - K * N;
-        for (int r = r0; r < r1; r++) s += dZ[(size_t)r * N + n];
+    float *out = part + (size_t)blockIdx.x * SG_NPARAM;
+    out[t] = g1;   // W1 [3][64], then b1
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        *reinterpret_cast<float4 *>(out + SG_OFF_W2 + (k0 + i) * SG_H + n) = g2[i];
+        *reinterpret_cast<float4 *>(out + SG_OFF_W3 + (k0 + i) * SG_H + n) = g3[i];
     }
-    part[(size_t)c * nq + q] = s;
+    if (k0 == 0) {
+        *reinterpret_cast<float4 *>(out + SG_OFF_B2 + n) = b2;
+        *reinterpret_cast<float4 *>(out + SG_OFF_B3 + n) = b3;
+    }
+    out[SG_OFF_W4 + t] = g4;
+    if (t < SG_OUT) out[SG_OFF_B4 + t] = b4;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
+    if ((t & 31) == 0) sm[TS_RED + (t >> 5)] = loss;
+    __syncthreads();
+    if (t == 0) {
+        float l = 0.f;
+        for (int w = 0; w < kTrainThreads / 32; w++) l += sm[TS_RED + w];
+        lossPart[blockIdx.x] = l;
+    }
+}
+static_assert(SG_OFF_B1 == SG_IN * SG_H && SG_H * (SG_IN + 1) == kTrainThreads && SG_H * SG_OUT == kTrainThreads &&
+                  (SG_H / 4) * (SG_H / 4) == kTrainThreads && kTrainS * SG_OUT * 2 == kTrainThreads,
+              "thread maps of k_sg_train");
+static_assert(SG_OFF_W2 % 4 == 0 && SG_OFF_B2 % 4 == 0 && SG_OFF_W3 % 4 == 0 && SG_OFF_B3 % 4 == 0 && SG_NPARAM % 4 == 0,
+              "16-byte gradient stores");
+
+struct AdamStep {
+    float lr, b1, b2, eps, c1, c2;
+};
+// G = sum of the blocks' gradients; with kAdam the parameter update.  64 parameters per block of 256
+// threads, each of 4 groups summing a quarter of the blocks: 2-3 us of dependent L2 reads instead of
+// 9 with one thread per parameter.
+constexpr int kReduceGroups = 4, kReduceParams = 64;
+template <bool kAdam>
+__global__ void __launch_bounds__(kReduceGroups *kReduceParams) k_sg_reduce(const float *__restrict__ part, int blocks,
+                                                                           float *P, float *G, float *M, float *V, AdamStep s) {
+    __shared__ float sh[kReduceGroups][kReduceParams];
+    const int lane = threadIdx.x % kReduceParams, grp = threadIdx.x / kReduceParams;
+    const int i = blockIdx.x * kReduceParams + lane;
+    const int per = (blocks + kReduceGroups - 1) / kReduceGroups;
+    const int lo = grp * per, hi = min(blocks, lo + per);
+    float a = 0.f;
+    if (i < SG_NPARAM) {
+#pragma unroll 8
+        for (int b = lo; b < hi; b++) a += part[(size_t)b * SG_NPARAM + i];
+    }
+    sh[grp][lane] = a;
+    __syncthreads();
+    if (grp || i >= SG_NPARAM) return;
+    const float g = ((sh[0][lane] + sh[1][lane]) + sh[2][lane]) + sh[3][lane];
+    G[i] = g;
+    if (kAdam) {
+        const float m = s.b1 * M[i] + (1.f - s.b1) * g;
+        const float v = s.b2 * V[i] + (1.f - s.b2) * g * g;
+        M[i] = m;
+        V[i] = v;
+        P[i] -= s.lr * (m / s.c1) / (sqrtf(v / s.c2) + s.eps);
+    }
 }
 
-// g[wOff + k*N+n] / g[bOff + n] = sum over chunks in order
-__global__ void k_reduce_chunks(const float *part, int chunks, int K, int N, float *g, int wOff, int bOff) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nq = K * N + N;
-    if (q >= nq) return;
-    float s = 0.f;
-    for (int c = 0; c < chunks; c++) s += part[(size_t)c * nq + q];
-    if (q < K * N) g[wOff + q] = s;
-    else g[bOff + (q - K * N)] = s;
-}
-
-__global__ void k_adam(float *P, const float *G, float *M, float *V, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
+// packed BF16 weights of the tensor-core layers from the FP32 parameters: one thread per element of a
+// layer's operand (N rows of K, K and N padded with zeros), in the canonical layout (tc_smem_off)
+__global__ void k_sg_pack(const float *__restrict__ P, unsigned char *__restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float g = G[i];
-    const float m = b1 * M[i] + (1.f - b1) * g;
-    const float v = b2 * V[i] + (1.f - b2) * g * g;
-    M[i] = m;
-    V[i] = v;
-    P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+    if (i >= TC_WBYTES / 2) return;
+    int wOff, K, N, rows, base;
+    if (i < TC_W2 / 2) { wOff = SG_OFF_W1; K = SG_IN; N = SG_H; rows = 64; base = TC_W1; }
+    else if (i < TC_W3 / 2) { wOff = SG_OFF_W2; K = SG_H; N = SG_H; rows = 64; base = TC_W2; }
+    else if (i < TC_W4 / 2) { wOff = SG_OFF_W3; K = SG_H; N = SG_H; rows = 64; base = TC_W3; }
+    else { wOff = SG_OFF_W4; K = SG_H; N = SG_OUT; rows = 16; base = TC_W4; }
+    const int q = i - base / 2, n = q % rows, k = q / rows;
+    const float w = (k < K && n < N) ? P[wOff + k * N + n] : 0.f;
+    *reinterpret_cast<__nv_bfloat16 *>(out + base + tc_smem_off(n, k, rows)) = __float2bfloat16_rn(w);
 }
 
 // batch prediction input: raw samples X[n][3]
@@ -174,25 +360,6 @@ struct InPredict {
 };
 
 // ---------------------------------------------------------------- host helpers
-uint16_t bf16_rne(float f) {
-    uint32_t u;
-    std::memcpy(&u, &f, 4);
-    if ((u & 0x7f800000u) == 0x7f800000u && (u & 0x007fffffu)) return (uint16_t)((u >> 16) | 0x40u);   // NaN
-    const uint32_t lsb = (u >> 16) & 1u;
-    u += 0x7fffu + lsb;
-    return (uint16_t)(u >> 16);
-}
-
-// one layer W[K][N] (row-major, in x out) as the B operand of the tensor-core layer: N rows of
-// K (K-major), K padded to 16 * kSlabs and N to nPad with zeros, in the canonical layout
-void pack_layer_tc(const float *W, int K, int N, int kSlabs, int nPad, unsigned char *out) {
-    for (int n = 0; n < nPad; n++)
-        for (int k = 0; k < 16 * kSlabs; k++) {
-            const uint16_t v = (k < K && n < N) ? bf16_rne(W[k * N + n]) : (uint16_t)0;
-            std::memcpy(out + tc_smem_off_host(n, k, nPad), &v, 2);
-        }
-}
-
 bool invert3(const double *a, double *inv) {
     const double det = a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) +
                        a[2] * (a[3] * a[7] - a[4] * a[6]);
@@ -223,77 +390,55 @@ struct fg_surrogate {
     bool hasNorm = false;
     // batch work buffers (capacity cap rows)
     int cap = 0;
-    Buf bx, by, z1, a1, z2, a2, z3, a3, yp, dy, d3, d2, d1, part, lossPart;
+    Buf bx, by;           // batch of fg_surrogate_loss_grad
+    Buf part, lossPart;   // per-block gradients and losses of a training pass
 
     int ensure_batch(int B) {
         if (B <= cap) return FG_OK;
-        cap = B;
-        const size_t h = (size_t)B * SG_H * sizeof(float);
         SG_TRY(bx.alloc((size_t)B * SG_IN * sizeof(float)));
         SG_TRY(by.alloc((size_t)B * SG_OUT * sizeof(float)));
-        for (Buf *b : {&z1, &a1, &z2, &a2, &z3, &a3, &d3, &d2, &d1}) SG_TRY(b->alloc(h));
-        SG_TRY(yp.alloc((size_t)B * SG_OUT * sizeof(float)));
-        SG_TRY(dy.alloc((size_t)B * SG_OUT * sizeof(float)));
-        SG_TRY(part.alloc((size_t)kChunks * (SG_H * SG_H + SG_H) * sizeof(float)));
-        SG_TRY(lossPart.alloc((size_t)((B * SG_OUT + 255) / 256) * sizeof(float)));
+        cap = B;
+        return FG_OK;
+    }
+    // work buffers of a training pass and its kernel's shared memory (above 48 KB), once
+    int ensure_train() {
+        if (part.p && lossPart.p) return FG_OK;
+        SG_TRY(cudaFuncSetAttribute(k_sg_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_END * (int)sizeof(float)));
+        SG_TRY(part.alloc((size_t)kTrainMaxBlocks * SG_NPARAM * sizeof(float)));
+        SG_TRY(lossPart.alloc(kTrainMaxBlocks * sizeof(float)));
         return FG_OK;
     }
 
     int repack() {
-        std::vector<float> p(SG_NPARAM);
-        SG_TRY(cudaMemcpy(p.data(), P.p, SG_NPARAM * sizeof(float), cudaMemcpyDeviceToHost));
-        std::vector<unsigned char> pk(TC_WBYTES, 0);
-        pack_layer_tc(p.data() + SG_OFF_W1, SG_IN, SG_H, 1, 64, pk.data() + TC_W1);
-        pack_layer_tc(p.data() + SG_OFF_W2, SG_H, SG_H, 4, 64, pk.data() + TC_W2);
-        pack_layer_tc(p.data() + SG_OFF_W3, SG_H, SG_H, 4, 64, pk.data() + TC_W3);
-        pack_layer_tc(p.data() + SG_OFF_W4, SG_H, SG_OUT, 4, 16, pk.data() + TC_W4);
-        SG_TRY(cudaMemcpy(pack.p, pk.data(), TC_WBYTES, cudaMemcpyHostToDevice));
+        k_sg_pack<<<(TC_WBYTES / 2 + 255) / 256, 256>>>(P.as<float>(), pack.as<unsigned char>());
+        SG_TRY(cudaGetLastError());
+        SG_TRY(cudaStreamSynchronize(0));
         return FG_OK;
     }
 
-    // forward + loss + backward over the batch in bx / by (standardised); grad into G
-    int fwd_bwd(int B, float *lossOut, cudaStream_t s) {
-        const float *Pp = P.as<float>();
-        float *Gp = G.as<float>();
-        const int T = 256;
-        auto grid = [&](long long c) { return (int)((c + T - 1) / T); };
-        k_dense_fwd<<<grid((long long)B * SG_H), T, 0, s>>>(bx.as<float>(), SG_IN, Pp + SG_OFF_W1, Pp + SG_OFF_B1, SG_H, B,
-                                                           z1.as<float>(), a1.as<float>(), 1);
-        k_dense_fwd<<<grid((long long)B * SG_H), T, 0, s>>>(a1.as<float>(), SG_H, Pp + SG_OFF_W2, Pp + SG_OFF_B2, SG_H, B,
-                                                           z2.as<float>(), a2.as<float>(), 1);
-        k_dense_fwd<<<grid((long long)B * SG_H), T, 0, s>>>(a2.as<float>(), SG_H, Pp + SG_OFF_W3, Pp + SG_OFF_B3, SG_H, B,
-                                                           z3.as<float>(), a3.as<float>(), 1);
-        k_dense_fwd<<<grid((long long)B * SG_OUT), T, 0, s>>>(a3.as<float>(), SG_H, Pp + SG_OFF_W4, Pp + SG_OFF_B4, SG_OUT,
-                                                             B, nullptr, yp.as<float>(), 0);
-        const int cnt = B * SG_OUT;
-        const int nLoss = grid(cnt);
-        k_sg_loss<<<nLoss, T, 0, s>>>(yp.as<float>(), by.as<float>(), cnt, 1.0f / (float)cnt, dy.as<float>(),
-                                      lossPart.as<float>());
-        const int chunk = (B + kChunks - 1) / kChunks;
-        auto wgrad = [&](const float *A, const float *dZ, int K, int N, int wOff, int bOff) {
-            dim3 g2(grid((long long)K * N + N), kChunks);
-            k_dense_bwd_w<<<g2, T, 0, s>>>(A, dZ, B, K, N, chunk, part.as<float>());
-            k_reduce_chunks<<<grid((long long)K * N + N), T, 0, s>>>(part.as<float>(), kChunks, K, N, Gp, wOff, bOff);
-        };
-        // layer 4 (linear): dZ4 = dy
-        wgrad(a3.as<float>(), dy.as<float>(), SG_H, SG_OUT, SG_OFF_W4, SG_OFF_B4);
-        k_dense_bwd_data<<<grid((long long)B * SG_H), T, 0, s>>>(dy.as<float>(), Pp + SG_OFF_W4, SG_OUT, SG_H,
-                                                                z3.as<float>(), B, d3.as<float>());
-        wgrad(a2.as<float>(), d3.as<float>(), SG_H, SG_H, SG_OFF_W3, SG_OFF_B3);
-        k_dense_bwd_data<<<grid((long long)B * SG_H), T, 0, s>>>(d3.as<float>(), Pp + SG_OFF_W3, SG_H, SG_H,
-                                                                z2.as<float>(), B, d2.as<float>());
-        wgrad(a1.as<float>(), d2.as<float>(), SG_H, SG_H, SG_OFF_W2, SG_OFF_B2);
-        k_dense_bwd_data<<<grid((long long)B * SG_H), T, 0, s>>>(d2.as<float>(), Pp + SG_OFF_W2, SG_H, SG_H,
-                                                                z1.as<float>(), B, d1.as<float>());
-        wgrad(bx.as<float>(), d1.as<float>(), SG_IN, SG_H, SG_OFF_W1, SG_OFF_B1);
+    // forward, loss and backward over B samples (rows perm[0 .. B) of x / y, standardised); the
+    // gradient goes into G, and with adam the parameters take the step
+    int fwd_bwd(const float *x, const float *y, const int32_t *rows, int B, const AdamStep *adam, float *lossOut, cudaStream_t s) {
+        const int rc = ensure_train();
+        if (rc != FG_OK) return rc;
+        const int blocks = std::min((B + kTrainS - 1) / kTrainS, kTrainMaxBlocks);
+        k_sg_train<<<blocks, kTrainThreads, TS_END * sizeof(float), s>>>(P.as<float>(), x, y, rows, B, 1.0f / (float)(B * SG_OUT),
+                                                                         part.as<float>(), lossPart.as<float>());
+        const int rb = (SG_NPARAM + kReduceParams - 1) / kReduceParams, rt = kReduceGroups * kReduceParams;
+        if (adam)
+            k_sg_reduce<true><<<rb, rt, 0, s>>>(part.as<float>(), blocks, P.as<float>(), G.as<float>(), M.as<float>(),
+                                                V.as<float>(), *adam);
+        else
+            k_sg_reduce<false><<<rb, rt, 0, s>>>(part.as<float>(), blocks, P.as<float>(), G.as<float>(), M.as<float>(),
+                                                 V.as<float>(), AdamStep{});
         SG_TRY(cudaGetLastError());
         if (lossOut) {
-            std::vector<float> lp(nLoss);
-            SG_TRY(cudaMemcpyAsync(lp.data(), lossPart.p, nLoss * sizeof(float), cudaMemcpyDeviceToHost, s));
+            float lp[kTrainMaxBlocks];
+            SG_TRY(cudaMemcpyAsync(lp, lossPart.p, blocks * sizeof(float), cudaMemcpyDeviceToHost, s));
             SG_TRY(cudaStreamSynchronize(s));
             double sum = 0;
-            for (float v : lp) sum += v;
-            *lossOut = (float)(sum / cnt);
+            for (int i = 0; i < blocks; i++) sum += lp[i];
+            *lossOut = (float)(sum / ((double)B * SG_OUT));
         }
         return FG_OK;
     }
@@ -427,8 +572,7 @@ int fg_surrogate_train(fg_surrogate *g, int32_t epochs, int32_t batch, float lr,
     if (epochs < 0 || batch < 32 || batch > (1 << 20) || !(lr > 0))
         return fg::set_error(FG_ERR_ARG, "fg_surrogate_train: epochs >= 0, 32 <= batch <= 2^20, lr > 0");
     SG_TRY(cudaSetDevice(g->device));
-    int rc = g->ensure_batch(batch);
-    if (rc != FG_OK) return rc;
+    int rc = FG_OK;
     cudaStream_t s = 0;
     std::mt19937_64 rng(seed);
     std::vector<int32_t> perm((size_t)g->n);
@@ -442,20 +586,17 @@ int fg_surrogate_train(fg_surrogate *g, int32_t epochs, int32_t batch, float lr,
         double sum = 0;
         // cosine decay of the learning rate over the whole run
         for (int64_t b = 0; b < nb; b++) {
-            k_sg_gather<<<(batch + 255) / 256, 256, 0, s>>>(g->perm.as<int32_t>(), (int)(b * batch), batch,
-                                                            g->X.as<float>(), g->Y.as<float>(), g->bx.as<float>(),
-                                                            g->by.as<float>());
             const bool last = (b == nb - 1);
             float l = 0;
-            rc = g->fwd_bwd(batch, last ? &l : nullptr, s);
-            if (rc != FG_OK) return rc;
-            if (last) sum = l;
             g->adamStep++;
             const double prog = ((double)ep * nb + b) / std::max<double>(1.0, (double)epochs * nb);
             const float lrt = (float)(lr * 0.5 * (1.0 + std::cos(3.14159265358979 * prog)));
             const float c1 = 1.f - std::pow(b1, (float)g->adamStep), c2 = 1.f - std::pow(b2, (float)g->adamStep);
-            k_adam<<<(SG_NPARAM + 255) / 256, 256, 0, s>>>(g->P.as<float>(), g->G.as<float>(), g->M.as<float>(),
-                                                          g->V.as<float>(), SG_NPARAM, lrt, b1, b2, eps, c1, c2);
+            const AdamStep adam{lrt, b1, b2, eps, c1, c2};
+            rc = g->fwd_bwd(g->X.as<float>(), g->Y.as<float>(), g->perm.as<int32_t>() + b * batch, batch, &adam,
+                            last ? &l : nullptr, s);
+            if (rc != FG_OK) return rc;
+            if (last) sum = l;
         }
         SG_TRY(cudaGetLastError());
         epochLoss = sum;
@@ -476,7 +617,7 @@ int fg_surrogate_loss_grad(fg_surrogate *g, const float *X, const float *Y, int3
     SG_TRY(cudaMemcpy(g->bx.p, X, (size_t)n * SG_IN * sizeof(float), cudaMemcpyHostToDevice));
     SG_TRY(cudaMemcpy(g->by.p, Y, (size_t)n * SG_OUT * sizeof(float), cudaMemcpyHostToDevice));
     float l = 0;
-    rc = g->fwd_bwd(n, &l, 0);
+    rc = g->fwd_bwd(g->bx.as<float>(), g->by.as<float>(), nullptr, n, nullptr, &l, 0);
     if (rc != FG_OK) return rc;
     SG_TRY(cudaMemcpy(grad, g->G.p, SG_NPARAM * sizeof(float), cudaMemcpyDeviceToHost));
     if (loss) *loss = l;
