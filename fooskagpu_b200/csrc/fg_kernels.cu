@@ -17,121 +17,77 @@
 
 #include <climits>
 
+
 namespace fg {
 
 
+// Face records (FREC values).  FP32: 48 consecutive bytes per face, three 16-byte vectors.  FP64: planes
+// of 16-byte vectors as the cell records: 96 consecutive bytes per face made every store and load
+// instruction of a warp touch 24 to 32 cache lines (96^3 TGV: face 355 -> 324 us, gather 133 -> 125 us;
+// 480 k tets: 124 -> 112, 67 -> 54 us); in FP32 planes cost the gather more than they save the face
+// kernel (128^3: face 292 -> 289, gather 202 -> 210 us).
 template <typename T>
-__device__ __forceinline__ void store_frec(T *FB, int f, const T *r) {
-    T *p = FB + (size_t)f * FREC;
-#pragma unroll
-    for (int v = 0; v < FREC; v++) p[v] = r[v];
-}
-template <>
-__device__ __forceinline__ void store_frec<float>(float *FB, int f, const float *r) {
-    float4 *p = reinterpret_cast<float4 *>(FB + (size_t)f * FREC);
-    p[0] = make_float4(r[0], r[1], r[2], r[3]);
-    p[1] = make_float4(r[4], r[5], r[6], r[7]);
-    p[2] = make_float4(r[8], r[9], r[10], r[11]);
+__device__ __forceinline__ void store_frec(T *FB, size_t nF, int f, const T *r) {
+    if constexpr (sizeof(T) == 8) {
+        rec_store<T, FREC>(FB, nF, f, r);
+    } else {
+        float4 *p = reinterpret_cast<float4 *>(FB + (size_t)f * FREC);
+        p[0] = make_float4(r[0], r[1], r[2], r[3]);
+        p[1] = make_float4(r[4], r[5], r[6], r[7]);
+        p[2] = make_float4(r[8], r[9], r[10], r[11]);
+    }
 }
 template <typename T>
-__device__ __forceinline__ void load_frec(const T *__restrict__ FB, int f, T *r) {
-    const T *p = FB + (size_t)f * FREC;
-#pragma unroll
-    for (int v = 0; v < FREC; v++) r[v] = __ldg(p + v);
-}
-template <>
-__device__ __forceinline__ void load_frec<float>(const float *__restrict__ FB, int f, float *r) {
-    const float4 *p = reinterpret_cast<const float4 *>(FB + (size_t)f * FREC);
-    const float4 a = __ldg(p), b = __ldg(p + 1), d = __ldg(p + 2);
-    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
-    r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
-    r[8] = d.x; r[9] = d.y; r[10] = d.z; r[11] = d.w;
+__device__ __forceinline__ void load_frec(const T *__restrict__ FB, size_t nF, int f, T *r) {
+    if constexpr (sizeof(T) == 8) {
+        rec_load<T, FREC>(FB, nF, f, r);
+    } else {
+        const float4 *p = reinterpret_cast<const float4 *>(FB + (size_t)f * FREC);
+        const float4 a = __ldg(p), b = __ldg(p + 1), d = __ldg(p + 2);
+        r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+        r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+        r[8] = d.x; r[9] = d.y; r[10] = d.z; r[11] = d.w;
+    }
 }
 
 // ------------------------------------------------------------------ shared-memory staging
-// A block handles `blockCells` consecutive (Morton-ordered, hence spatially compact) cells.  It
-// first copies into shared memory
-//   - the records of its own cells and of its halo (face neighbours outside the block),
-//   - the per-slot face geometry of its own cells (contiguous in the cell-major layout),
-// then each thread computes its cell's faces from shared memory only.  Strides are odd numbers
-// of words so that threads of a warp reading the same field of consecutive cells hit distinct
-// banks.  slotLocal holds the neighbour's staged-record index, or -bc on a boundary slot.
-constexpr int kGeoComp = 6;    // aox aoy aoz dcx dcy dcz
+// The gradient kernel gives a block a brick of consecutive (Morton-ordered, hence spatially compact)
+// cells.  The block first copies the records of the brick's cells and of its halo (the
+// neighbours outside it) into shared memory, in planes of 16-byte vectors as in global memory
+// (vector q of staged record r at sm[q * rows + r]), with asynchronous copies; every face then reads
+// its two records from there.
+__device__ __forceinline__ void cp_async16(void *smem, const void *g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// record area rounded up to 16 bytes so the staged geometry arrays start aligned
 template <typename T>
-__host__ __device__ inline size_t rec_area(const DevMesh<T> &m, int stride) {
-    return (((size_t)(m.blockCells + m.maxHalo) * stride * sizeof(T)) + 15) / 16 * 16;
+__host__ __device__ constexpr int stage_w_vecs() { return (NP + vpv<T>() - 1) / vpv<T>(); }
+template <typename T>
+constexpr size_t grad_smem(int rows) { return (size_t)rows * stage_w_vecs<T>() * 16; }
+
+// NVAL values of staged record r from the planes of 16-byte vectors starting at plane q0
+template <typename T, int NVAL>
+__device__ __forceinline__ void staged_load(const typename Vec16<T>::type *sm, int rows, int q0, int r, T *out) {
+    constexpr int P = vpv<T>();
+#pragma unroll
+    for (int q = 0; q < (NVAL + P - 1) / P; q++) {
+        const typename Vec16<T>::type x = sm[(q0 + q) * rows + r];
+#pragma unroll
+        for (int j = 0; j < P; j++)
+            if (q * P + j < NVAL) out[q * P + j] = vlane(x, j);
+    }
 }
 
-template <typename T> struct Stage;
-template <> struct Stage<float> {
-    static constexpr int WS = 13;   // W(9) + volume + pad, odd
-};
-template <> struct Stage<double> {
-    static constexpr int WS = 11;
-};
-__host__ __device__ constexpr int slot_stride(int nSlots) { return nSlots | 1; }
-
-// per-slot geometry of a cell: staged in shared memory, or read from global memory
+// two consecutive values of a per-slot array
+template <typename T> struct Pair;
+template <> struct Pair<float> { using type = float2; };
+template <> struct Pair<double> { using type = double2; };
 template <typename T>
-struct SlotGeo {
-    const T *sg;
-    const int *sl;
-    int GS;         // component stride of the staged arrays
-    int d0;         // t * slot stride
-    const DevMesh<T> *m;
-    size_t g0;      // c * nSlots
-    __device__ __forceinline__ T get(int comp, int k) const {
-#if FG_STAGE_GEOMETRY
-        return sg[comp * GS + d0 + k];   // d0 = t * nSlots
-#else
-        const size_t g = g0 + k;
-        switch (comp) {
-        case 0: return m->aox[g];
-        case 1: return m->aoy[g];
-        case 2: return m->aoz[g];
-        case 3: return m->dcx[g];
-        case 4: return m->dcy[g];
-        default: return m->dcz[g];
-        }
-#endif
-    }
-    __device__ __forceinline__ int local(int k) const {
-#if FG_STAGE_GEOMETRY
-        return sl[d0 + k];
-#else
-        return m->slotLocal[g0 + k];
-#endif
-    }
-};
-
-template <typename T>
-__device__ __forceinline__ int staged_source(const DevMesh<T> &m, int b, int r, int lo, int nOwn) {
-    return (r < m.blockCells) ? ((r < nOwn) ? lo + r : -1) : m.haloIds[m.haloStart[b] + (r - m.blockCells)];
-}
-
-// copy the per-slot geometry and local indices of the block's own cells: the block's slots are a
-// contiguous range of each cell-major array, copied with 16-byte loads in the global layout
-template <typename T>
-__device__ __forceinline__ void stage_geometry(const DevMesh<T> &m, int lo, int nOwn, T *sg, int *sl) {
-#if !FG_STAGE_GEOMETRY
-    return;
-#endif
-    using V = typename Vec16<T>::type;
-    constexpr int TPV = 16 / sizeof(T);
-    const int S = m.nSlots;
-    const int B = m.blockCells;
-    const int nV = (nOwn * S + TPV - 1) / TPV;          // vectors per component actually used
-    const int stride = B * S;                            // component stride in shared memory
-    const size_t cstride = m.geoStride;
-    const size_t g0 = (size_t)lo * S;                    // 16-byte aligned: B * S * sizeof(T) % 16 == 0
-    for (int i = threadIdx.x; i < kGeoComp * nV; i += blockDim.x) {
-        const int cpt = i / nV, j = i % nV;
-        const V x = __ldg(reinterpret_cast<const V *>(m.aox + cpt * cstride + g0) + j);
-        reinterpret_cast<V *>(sg + (size_t)cpt * stride)[j] = x;
-    }
-    for (int i = threadIdx.x; i < nOwn * S; i += blockDim.x) sl[i] = m.slotLocal[g0 + i];
+__device__ __forceinline__ void load_pair(const T *__restrict__ p, T *out) {
+    const typename Pair<T>::type x = __ldg(reinterpret_cast<const typename Pair<T>::type *>(p));
+    out[0] = x.x;
+    out[1] = x.y;
 }
 
 // ------------------------------------------------------------------ gradient + limiter
@@ -146,95 +102,87 @@ __device__ __forceinline__ T limiter_phi(T num, T diff) {
     return num / (2 * diff);
 }
 
-// slot loops of the gradient kernel: unrolled to the largest face count (the loads of every slot
-// can then be issued early), or a plain loop to the cell's face count
-#ifndef FG_GRAD_UNROLL
-#define FG_GRAD_UNROLL 1
-#endif
-#if FG_GRAD_UNROLL
-#define FG_GRAD_SLOT_LOOP(k, nf) _Pragma("unroll") for (int k = 0; k < MAXSLOT; k++) if (k < (nf))
-#else
-#define FG_GRAD_SLOT_LOOP(k, nf) for (int k = 0; k < (nf); k++)
-#endif
-
-// kLim: 0 the reference's limiter function, 1 the van Albada-type extension (fg_case.limiter)
-template <typename T, int kLim>
+// kLim: 0 the reference's limiter function, 1 the van Albada-type extension (fg_case.limiter); S: slots
+// per cell (4: tets only, 6).  The two slot loops run over pairs of slots, whose geometry is one
+// 8-byte (FP64: 16-byte) load per component: the per-slot arrays are cell-major, so a scalar load per
+// slot touches the same cache lines S times over.  Bound by latency (staging, then the geometry).
+// Measured against scalar loads and records staged value by value: FP32 196 -> 177 us (128^3 hexes),
+// 86 -> 78 (981 k tets); FP64 224 -> 213 (96^3 hexes), 123 -> 109 (480 k tets).
+template <typename T, int kLim, int S>
 __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_grad(const DevMesh<T> m, const T *__restrict__ W,
                                                                 T *__restrict__ G, const PhysT<T> P) {
-    constexpr int WS = Stage<T>::WS;
+    using V = typename Vec16<T>::type;
+    constexpr int B = StageCells<T>::value, WQ = stage_w_vecs<T>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    V *sm = reinterpret_cast<V *>(smem_raw);
     const int b = blockIdx.x;
-    const int B = m.blockCells;
     const int lo = b * B;
-    const int nOwn = min(B, m.nG - lo);      // cells whose gradients this block computes
+    const int nOwn = min(B, m.nG - lo);       // cells whose gradients this block computes
     const int nBlockRecs = min(B, m.n - lo);  // cells of the block range with records (ghosts of a part too)
-    const int nRec = B + (m.haloStart[b + 1] - m.haloStart[b]);
-    const int SS = slot_stride(m.nSlots);
-    T *rec = reinterpret_cast<T *>(smem_raw);                       // nRecMax * WS
-    T *sg = reinterpret_cast<T *>(smem_raw + rec_area<T>(m, WS));   // kGeoComp * B * nSlots
-    int *sl = reinterpret_cast<int *>(sg + (size_t)kGeoComp * B * m.nSlots);
-    {
-        // each lane copies one 16-byte vector of a W record; consecutive lanes take the same
-        // vector of consecutive staged cells (contiguous for the block's own cells)
-        using V = typename Vec16<T>::type;
-        constexpr int TPV = vpv<T>();
-        constexpr int WV = (NP + TPV - 1) / TPV;   // vectors holding the NP used values
-        const V *Wv = reinterpret_cast<const V *>(W);
-        for (int r = threadIdx.x; r < nRec; r += blockDim.x) {
-            const int src = staged_source(m, b, r, lo, nBlockRecs);
-            if (src < 0) continue;
+    const int rows = B + m.maxHalo;
+    const int hs = m.haloStart[b], nRec = B + (m.haloStart[b + 1] - hs);
+    for (int r = threadIdx.x; r < nRec; r += B) {
+        if (r < B && r >= nBlockRecs) continue;
+        const int src = r < B ? lo + r : m.haloIds[hs + r - B];
 #pragma unroll
-            for (int q = 0; q < WV; q++) {
-                const V x = __ldg(Wv + (size_t)q * m.n + src);
-#pragma unroll
-                for (int j = 0; j < TPV; j++)
-                    if (q * TPV + j < NP) rec[r * WS + q * TPV + j] = vlane(x, j);
-            }
-        }
+        for (int q = 0; q < WQ; q++) cp_async16(sm + q * rows + r, reinterpret_cast<const V *>(W) + (size_t)q * m.n + src);
     }
-    stage_geometry(m, lo, nOwn, sg, sl);
-    __syncthreads();
     const int t = threadIdx.x;
     const int c = lo + t;
-    if (t >= nOwn) return;
-    const SlotGeo<T> geo{sg, sl, B * m.nSlots, t * m.nSlots, &m, (size_t)c * m.nSlots};
+    const bool own = t < nOwn;
+    const int fl = own ? m.flags[c] : 0;
+    const T iv = own ? (T)m.ivol[c] : (T)0;
+    cp_async_wait();
+    __syncthreads();
+    if (!own) return;
+    const size_t g0 = (size_t)c * S;
     T w[NP], gs[NP * 3], mn[NP], mx[NP];
+    staged_load<T, NP>(sm, rows, 0, t, w);
 #pragma unroll
     for (int v = 0; v < NP; v++) {
-        w[v] = rec[t * WS + v];
         gs[3 * v] = gs[3 * v + 1] = gs[3 * v + 2] = 0;
         mn[v] = (T)1e12;
         mx[v] = (T)-1e12;
     }
-    const int fl = m.flags[c];
     const int nf = fl & 7;
-    FG_GRAD_SLOT_LOOP(k, nf) {
-        const int li = geo.local(k);
-        // outward n A of the face (the host computed (+-1) n A in T arithmetic, as the reference's
-        // sign times normal times area)
-        const T ax = geo.get(0, k), ay = geo.get(1, k), az = geo.get(2, k);
-        T ot[NP];
-        if (li >= 0) {
 #pragma unroll
-            for (int v = 0; v < NP; v++) ot[v] = rec[li * WS + v];
-        } else {
-            // boundary slot: the cell owns the face, so its canonical normal points outward
-            const int fi = m.slotFace[(size_t)c * m.nSlots + k];
+    for (int k2 = 0; k2 < S; k2 += 2) {
+        if (k2 >= nf) break;
+        T ax[2], ay[2], az[2];
+        load_pair(m.aox + g0 + k2, ax);
+        load_pair(m.aoy + g0 + k2, ay);
+        load_pair(m.aoz + g0 + k2, az);
+        const int sl = __ldg(reinterpret_cast<const int *>(m.slotLocal + g0 + k2));
 #pragma unroll
-            for (int v = 0; v < NP; v++) ot[v] = w[v];
-            ghost_state(P, -li, m.fnx[fi], m.fny[fi], m.fnz[fi], ot);
-        }
+        for (int j = 0; j < 2; j++) {
+            const int k = k2 + j;
+            if (k >= nf) break;
+            const int li = j ? sl >> 16 : (int)(int16_t)sl;
+            // half the outward n A of the face (the host computed (+-1) n A in T arithmetic, as the
+            // reference's sign times normal times area): (w + w_nb) times it is exactly the mean
+            // times the whole
+            const T hx = ax[j] * (T)0.5, hy = ay[j] * (T)0.5, hz = az[j] * (T)0.5;
+            T ot[NP];
+            if (li >= 0) {
+                staged_load<T, NP>(sm, rows, 0, li, ot);
+            } else {
+                // boundary slot: the cell owns the face, so its canonical normal points outward
+                const int fi = m.slotFace[g0 + k];
 #pragma unroll
-        for (int v = 0; v < NP; v++) {
-            mx[v] = fmax(mx[v], ot[v]);
-            mn[v] = fmin(mn[v], ot[v]);
-            const T h = (w[v] + ot[v]) * (T)0.5;
-            gs[3 * v + 0] += h * ax;
-            gs[3 * v + 1] += h * ay;
-            gs[3 * v + 2] += h * az;
+                for (int v = 0; v < NP; v++) ot[v] = w[v];
+                ghost_state(P, -li, m.fnx[fi], m.fny[fi], m.fnz[fi], ot);
+            }
+#pragma unroll
+            for (int v = 0; v < NP; v++) {
+                mx[v] = fmax(mx[v], ot[v]);
+                mn[v] = fmin(mn[v], ot[v]);
+                const T h = w[v] + ot[v];
+                gs[3 * v + 0] += h * hx;
+                gs[3 * v + 1] += h * hy;
+                gs[3 * v + 2] += h * hz;
+            }
         }
     }
-    const T iv = (T)(1.0 / m.vol[c]);
 #pragma unroll
     for (int q = 0; q < NP * 3; q++) gs[q] *= iv;
     // limiter (DP/computeFaceValues.cu:66-81): theta = min over the faces of clamp(phi, 0, 1), phi
@@ -246,14 +194,23 @@ __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_gr
     T dpos[NP], dneg[NP];
 #pragma unroll
     for (int v = 0; v < NP; v++) dpos[v] = dneg[v] = 0;
-    FG_GRAD_SLOT_LOOP(k, nf) {
-        const T dx = geo.get(3, k), dy = geo.get(4, k), dz = geo.get(5, k);
 #pragma unroll
-        for (int v = 0; v < NP; v++) {
-            const T ext = dx * gs[3 * v] + dy * gs[3 * v + 1] + dz * gs[3 * v + 2];
-            const T diff = (w[v] + ext) - w[v];
-            dpos[v] = fmax(dpos[v], diff);
-            dneg[v] = fmin(dneg[v], diff);
+    for (int k2 = 0; k2 < S; k2 += 2) {
+        if (k2 >= nf) break;
+        T dx[2], dy[2], dz[2];
+        load_pair(m.dcx + g0 + k2, dx);
+        load_pair(m.dcy + g0 + k2, dy);
+        load_pair(m.dcz + g0 + k2, dz);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            if (k2 + j >= nf) break;
+#pragma unroll
+            for (int v = 0; v < NP; v++) {
+                const T ext = dx[j] * gs[3 * v] + dy[j] * gs[3 * v + 1] + dz[j] * gs[3 * v + 2];
+                const T diff = (w[v] + ext) - w[v];
+                dpos[v] = fmax(dpos[v], diff);
+                dneg[v] = fmin(dneg[v], diff);
+            }
         }
     }
     T th[NP];
@@ -300,7 +257,7 @@ __device__ __forceinline__ void cell_grad_t(const PhysT<T> &P, const T *w, const
 template <typename T>
 __device__ __forceinline__ T face_tail(const PhysT<T> &P, const T *sL, const T *sR, const T *p1, const T *gO,
                                           const T *gN, const T *gT, int nb, T nx, T ny, T nz, T A, T lsSq,
-                                          int wantSignal, T *__restrict__ FB, int fi) {
+                                          int wantSignal, T *__restrict__ FB, size_t nF, int fi) {
     T F[NV], unc, pF;
     hllc_flux(P, sL, sR, nx, ny, nz, F, unc, pF);
     T H[NV];
@@ -349,7 +306,7 @@ __device__ __forceinline__ T face_tail(const PhysT<T> &P, const T *sL, const T *
     for (int v = 0; v < NV; v++) rec[v] = H[v];
     rec[NV] = A * unc;
     rec[NV + 1] = sig;
-    store_frec(FB, fi, rec);
+    store_frec(FB, nF, fi, rec);
     return sig;
 }
 
@@ -415,7 +372,7 @@ __global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(co
 #pragma unroll
         for (int q = 0; q < 9; q++) gN[q] = gO[q];
     }
-    const T sig = face_tail(P, sL, sR, p1, gO, gN, gT, nb, nx, ny, nz, A, m.fLsSq[fi], wantSignal, FB, fi);
+    const T sig = face_tail(P, sL, sR, p1, gO, gN, gT, nb, nx, ny, nz, A, m.fLsSq[fi], wantSignal, FB, (size_t)m.nF, fi);
     if (wantSignal == 2) {
         // own cells only: a ghost's dt bound belongs to its own part
         if (o < m.nU) signal_max(cellSig + o, sig);
@@ -424,7 +381,29 @@ __global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(co
 }
 
 // ------------------------------------------------------------------ owner-side gather + RK
-template <typename T>
+// the face ids of a cell's S slots
+template <int S>
+__device__ __forceinline__ void load_slot_faces(const int32_t *__restrict__ p, int *id) {
+    if constexpr (S == 4) {
+        const int4 x = __ldg(reinterpret_cast<const int4 *>(p));
+        id[0] = x.x;
+        id[1] = x.y;
+        id[2] = x.z;
+        id[3] = x.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < S; k += 2) {
+            const int2 x = __ldg(reinterpret_cast<const int2 *>(p + k));
+            id[k] = x.x;
+            id[k + 1] = x.y;
+        }
+    }
+}
+
+// S: slots per cell (4 or 6).  The face ids of all slots come first, in 8- or 16-byte loads, so that the
+// record of a face does not wait for its id in turn (with the fewer divisions of cons2prim_d, FP64 96^3
+// TGV: 165 -> 133 us; FP32 is bound by memory at 128^3, 201 us, and by this chain on few cells).
+template <typename T, int S>
 __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gather(const DevMesh<T> m, Fields<T> f, const PhysD D, int mode,
                                                 int wantSignal, StageCoef sc) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -437,12 +416,15 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
 #pragma unroll
         for (int v = 0; v < NV; v++) acc[v] = 0.0;
         T sig = (T)-1e9;
-        const size_t base = (size_t)c * m.nSlots;
-        for (int k = 0; k < nf; k++) {
-            const int fi = m.slotFace[base + k];
+        int id[S];
+        load_slot_faces<S>(m.slotFace + (size_t)c * S, id);
+#pragma unroll
+        for (int k = 0; k < S; k++) {
+            if (k >= nf) break;
+            const int fi = id[k];
             const double s = ((fl >> (3 + k)) & 1) ? -1.0 : 1.0;
             T rec[FREC];
-            load_frec(f.FB, fi, rec);
+            load_frec(f.FB, (size_t)m.nF, fi, rec);
 #pragma unroll
             for (int v = 0; v < NV; v++) acc[v] += s * (double)rec[v];
             su += s * (double)rec[NV];
@@ -458,7 +440,6 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
         acc[3] += pc * (double)m.closure[c];
         acc[4] += pc * (double)m.closure[(size_t)m.n + c];
         acc[5] += pc * (double)m.closure[2 * (size_t)m.n + c];
-        const double vc = m.vol[c];
         if (wantSignal) {
             f.signal[c] = (double)sig;
             cfl = m.volP[c] / (double)sig;
@@ -468,8 +449,8 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
             for (int v = 0; v < NV; v++) f.RHS[(size_t)v * n + c] = acc[v];
         } else {
             // FP64 Runge-Kutta combination (DP/update.cu:19-103)
-            const double dt = *f.dt;
-            const double dtv = dt * (1.0 / vc);
+            const double dt = *f.dt, iv = m.ivol[c];
+            const double dtv = dt * iv;
             double u[NV];
 #pragma unroll
             for (int v = 0; v < NV; v++) {
@@ -483,9 +464,9 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
                     const double u0 = sc.writeU0 ? uc : f.U0[q];
                     r = u0 + dtv * acc[v];
                 } else if (sc.irk == 1) {
-                    r = 0.75 * f.U0[q] + 0.25 * uc + (0.25 * dt) * (1.0 / vc) * acc[v];
+                    r = 0.75 * f.U0[q] + 0.25 * uc + (0.25 * dt) * iv * acc[v];
                 } else {
-                    r = (1.0 / 3.0) * f.U0[q] + (2.0 / 3.0) * uc + ((2.0 / 3.0) * dt) * (1.0 / vc) * acc[v];
+                    r = (1.0 / 3.0) * f.U0[q] + (2.0 / 3.0) * uc + ((2.0 / 3.0) * dt) * iv * acc[v];
                 }
                 if (v == 5 && sc.neglectZ) r = 0.0;
                 u[v] = r;
@@ -543,19 +524,19 @@ __global__ void k_update(const DevMesh<T> m, Fields<T> f, const PhysD D, StageCo
     const int n = m.nU;
     if (c >= n) return;
     const double dt = *f.dt;
-    const double vc = m.vol[c];
+    const double iv = m.ivol[c];
     double u[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) {
         const size_t q = (size_t)v * n + c;
         const double uc = f.U[q], R = f.RHS[q];
         double r;
-        if (sc.rk == 1) r = uc + dt * (1.0 / vc) * R;
+        if (sc.rk == 1) r = uc + dt * iv * R;
         else if (sc.irk == 0) {
             if (sc.writeU0) f.U0[q] = uc;
-            r = (sc.writeU0 ? uc : f.U0[q]) + dt * (1.0 / vc) * R;
-        } else if (sc.irk == 1) r = 0.75 * f.U0[q] + 0.25 * uc + (0.25 * dt) * (1.0 / vc) * R;
-        else r = (1.0 / 3.0) * f.U0[q] + (2.0 / 3.0) * uc + ((2.0 / 3.0) * dt) * (1.0 / vc) * R;
+            r = (sc.writeU0 ? uc : f.U0[q]) + dt * iv * R;
+        } else if (sc.irk == 1) r = 0.75 * f.U0[q] + 0.25 * uc + (0.25 * dt) * iv * R;
+        else r = (1.0 / 3.0) * f.U0[q] + (2.0 / 3.0) * uc + ((2.0 / 3.0) * dt) * iv * R;
         if (v == 5 && sc.neglectZ) r = 0.0;
         u[v] = r;
         f.U[q] = r;
@@ -768,16 +749,6 @@ constexpr int kGatherThreads = FG_GATHER_THREADS;
 int flux_blocks(int n) { return (n + kGatherThreads - 1) / kGatherThreads; }
 int cons_blocks(int n) { return (n + kConsThreads - 1) / kConsThreads; }
 
-template <typename T>
-static size_t geo_smem(const DevMesh<T> &m) {
-    if (!FG_STAGE_GEOMETRY) return 0;
-    const size_t slots = (size_t)m.blockCells * m.nSlots;
-    return slots * kGeoComp * sizeof(T) + slots * sizeof(int);
-}
-template <typename T>
-static size_t grad_smem(const DevMesh<T> &m) {
-    return rec_area<T>(m, Stage<T>::WS) + geo_smem(m);
-}
 // raise (never lower) a kernel's dynamic shared-memory limit on the current device: solvers of
 // different meshes launch the same kernels with different amounts
 static int raise_smem(const void *fn, size_t bytes) {
@@ -788,15 +759,17 @@ static int raise_smem(const void *fn, size_t bytes) {
 }
 template <typename T>
 int stage_kernels_setup(const DevMesh<T> &m) {
-    return raise_smem((const void *)k_grad<T, 0>, grad_smem(m)) | raise_smem((const void *)k_grad<T, 1>, grad_smem(m));
+    const size_t gb = grad_smem<T>(m.blockCells + m.maxHalo);
+    return raise_smem((const void *)k_grad<T, 0, 4>, gb) | raise_smem((const void *)k_grad<T, 1, 4>, gb) |
+           raise_smem((const void *)k_grad<T, 0, 6>, gb) | raise_smem((const void *)k_grad<T, 1, 6>, gb);
 }
 template <typename T>
 void launch_grad(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, cudaStream_t s) {
     const int nb = (m.nG + m.blockCells - 1) / m.blockCells;
-    if (P.limiter == 1)
-        k_grad<T, 1><<<nb, m.blockCells, grad_smem(m), s>>>(m, f.Win, f.G, P);
-    else
-        k_grad<T, 0><<<nb, m.blockCells, grad_smem(m), s>>>(m, f.Win, f.G, P);
+    const size_t sm = grad_smem<T>(m.blockCells + m.maxHalo);
+    auto *k = m.nSlots == 4 ? (P.limiter == 1 ? k_grad<T, 1, 4> : k_grad<T, 0, 4>)
+                            : (P.limiter == 1 ? k_grad<T, 1, 6> : k_grad<T, 0, 6>);
+    k<<<nb, m.blockCells, sm, s>>>(m, f.Win, f.G, P);
 }
 template <typename T>
 void launch_face(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, int wantSignal, cudaStream_t s) {
@@ -811,7 +784,8 @@ void launch_cell_cfl(const DevMesh<T> &m, const Fields<T> &f, cudaStream_t s) {
 template <typename T>
 void launch_gather(const DevMesh<T> &m, const Fields<T> &f, const PhysD &D, int mode, int wantSignal,
                    StageCoef sc, cudaStream_t s) {
-    k_gather<T><<<flux_blocks(m.nU), kGatherThreads, 0, s>>>(m, f, D, mode, wantSignal, sc);
+    auto *k = m.nSlots == 4 ? k_gather<T, 4> : k_gather<T, 6>;
+    k<<<flux_blocks(m.nU), kGatherThreads, 0, s>>>(m, f, D, mode, wantSignal, sc);
 }
 template int stage_kernels_setup<float>(const DevMesh<float> &);
 template int stage_kernels_setup<double>(const DevMesh<double> &);

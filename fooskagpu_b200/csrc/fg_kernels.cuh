@@ -12,7 +12,7 @@ struct DevMesh {
     int nU;             // own cells: the first nU cells carry a state (U, U0, RHS rows) and are updated
     int nG;             // cells with gradients: own cells, then a part's first-layer ghosts
     int nFEval;         // faces the face kernel evaluates (those touching an own cell) come first
-    int nSlots;         // max faces per cell
+    int nSlots;         // slots per cell: 4 (tets only) or 6
     const int32_t *nbr;   // neighbour cell, or -bc (1..5) on a boundary slot, or INT32_MIN unused
     const int32_t *flags; // bits 0-2: faces of the cell; bit 3+k: cell owns the face of slot k
     // the six per-slot geometry arrays below are consecutive blocks of geoStride values, in this
@@ -22,6 +22,7 @@ struct DevMesh {
     const T *aox, *aoy, *aoz;        // outward area vector of the slot's face seen from the cell, n A
     const T *dcx, *dcy, *dcz;        // face centre - own cell centre
     const double *vol;               // cell volume
+    const double *ivol;              // 1 / vol
     const double *volP;              // pow(vol, 0.3333) as the reference's CFL bound uses
     // shared-memory staging: blocks of `blockCells` consecutive cells; the face neighbours of a
     // block that lie outside it (its halo) are listed in haloIds[haloStart[b] .. haloStart[b+1]);
@@ -57,11 +58,6 @@ constexpr int FREC = 12;
 #ifndef FG_STAGE_CELLS_D
 #define FG_STAGE_CELLS_D 64
 #endif
-// 1: the per-slot geometry of a block is staged in shared memory with its records;
-// 0: each face reads its geometry from global memory
-#ifndef FG_STAGE_GEOMETRY
-#define FG_STAGE_GEOMETRY 0
-#endif
 // owner cells per tile of the GPU face order (1: by owner cell, then slot).  Tiles of 32 measured
 // 1-3 % faster per step than 1 on the 128^3 hex workload (the gather reads nearby records) and
 // within 1 % on the graded tet ball.
@@ -70,10 +66,11 @@ constexpr int FREC = 12;
 #endif
 constexpr int kFaceTile = FG_FACE_TILE;
 // Minimum resident blocks per SM asked of the compiler (its register budget).  The FP32 stage
-// kernels are latency-bound gathers: capping registers at 85 / 85 / 51 per thread (gradient,
-// face, gather) raises the warps in flight and measured 2-9 % faster on the 128^3 hex workload.  The
-// FP64 gradient and gather kernels need their registers (capping them spills): 0 leaves the choice
-// to the compiler.
+// kernels are latency-bound gathers: capping registers at 96 / 80 / 48 per thread (gradient,
+// face, gather) raises the warps in flight.  Gradient on 128^3 hexes: 178 us at 6 blocks (80 registers,
+// 96 bytes of spill), 177 at 5, 202 at 4; on 981 k tets 80, 78, 78.  FP64 gradient (64 threads): 6 blocks
+// (168 registers) 213 us on 96^3 hexes, uncapped (188) 267, 7 blocks 267.  0 leaves the choice to the
+// compiler (FP64 gather).
 #ifndef FG_FACE_THREADS
 #define FG_FACE_THREADS 64
 #endif
@@ -81,7 +78,7 @@ constexpr int kFaceTile = FG_FACE_TILE;
 #define FG_GATHER_THREADS 128
 #endif
 #ifndef FG_GRAD_MINB
-#define FG_GRAD_MINB 6
+#define FG_GRAD_MINB 5
 #endif
 #ifndef FG_FACE_MINB
 #define FG_FACE_MINB (6 * 128 / FG_FACE_THREADS)
@@ -93,7 +90,7 @@ template <typename T> struct MinBlocks {
     static constexpr int grad = FG_GRAD_MINB, face = FG_FACE_MINB, gather = FG_GATHER_MINB;
 };
 #ifndef FG_GRAD_MINB_D
-#define FG_GRAD_MINB_D 0
+#define FG_GRAD_MINB_D 6
 #endif
 // FP64 face kernel: 6 resident blocks of 64 (168 registers, 88 bytes of spill) measured 15 % faster
 // than the compiler's 200 registers (5 blocks) on the 128^3 hex workload

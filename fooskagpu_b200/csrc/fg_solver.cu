@@ -291,7 +291,7 @@ constexpr int kSparseChemInv = 10;
 
 template <typename T>
 struct SolverT : public fg_solver {
-    DevBuf dNbr, dFlags, dGeo, dVol, dVolP, dNew2Old, dHaloStart, dHaloIds, dSlotLocal;
+    DevBuf dNbr, dFlags, dGeo, dVol, dVolP, dIVol, dNew2Old, dHaloStart, dHaloIds, dSlotLocal;
     DevBuf dU, dU0, dRHS, dW[2], dG, dSig, dCellSig, dBlockMin, dScal, dCnt, dCons, dStage;
     DevBuf dStageIn;   // staging buffer of the asynchronous uploads (on first use)
     DevBuf dStageOut[2];   // staging buffers of the asynchronous downloads (on first use)
@@ -331,7 +331,8 @@ struct SolverT : public fg_solver {
         nU = m.owned();
         nG = m.gradient_cells();
         parted = m.nOwned >= 0;
-        nSlots = m.maxFaces;
+        // even, so that the kernels load the per-slot arrays in pairs
+        nSlots = m.maxFaces <= 4 ? 4 : MAXSLOT;
         cellCenter.assign(m.cellCenter.begin(), m.cellCenter.end());
         FG_CUDA_TRY(cudaSetDevice(device));
         if (init_flag() != FG_OK) return FG_ERR_CUDA;
@@ -426,11 +427,12 @@ struct SolverT : public fg_solver {
         const size_t GS = (S * sizeof(T) + 15) / 16 * 16 / sizeof(T);
         std::vector<int32_t> nbr(S, INT32_MIN), flags(n, 0);
         std::vector<T> geo(6 * GS, (T)0);
-        std::vector<double> volP(n), vol(n);
+        std::vector<double> volP(n), vol(n), ivol(n);
         for (int i = 0; i < n; i++) {
             const int o = m.new2old[i];
             const fg::ElemType *et = fg::elem_type_for_nodes(m.elNN[o]);
             vol[i] = m.volume[o];
+            ivol[i] = 1.0 / m.volume[o];
             volP[i] = pow(m.volume[o], 0.3333);
             if (i >= nG) continue;   // a second-layer ghost: records only, no faces of its own
             int fl = et->nFaces;
@@ -587,6 +589,8 @@ struct SolverT : public fg_solver {
         FG_CUDA_TRY(dGeo.alloc(6 * GS * sizeof(T)));
         FG_CUDA_TRY(dVol.alloc((size_t)n * sizeof(double)));
         FG_CUDA_TRY(dVolP.alloc((size_t)n * sizeof(double)));
+        FG_CUDA_TRY(dIVol.alloc((size_t)n * sizeof(double)));
+        FG_CUDA_TRY(cudaMemcpy(dIVol.p, ivol.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(dNew2Old.alloc((size_t)n * sizeof(int32_t)));
         FG_CUDA_TRY(cudaMemcpy(dNbr.p, nbr.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dFlags.p, flags.data(), (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -595,11 +599,13 @@ struct SolverT : public fg_solver {
         FG_CUDA_TRY(cudaMemcpy(dVolP.p, volP.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dNew2Old.p, m.new2old.data(), (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(dFIdx.alloc(2 * (size_t)nF * sizeof(int32_t)));
+        FG_CUDA_TRY(cudaMemcpy(dFIdx.p, fIdx.data(), 2 * (size_t)nF * sizeof(int32_t), cudaMemcpyHostToDevice));
+        dm.fOwn = dFIdx.as<int32_t>();
+        dm.fNb = dFIdx.as<int32_t>() + nF;
         FG_CUDA_TRY(dFGeo.alloc(11 * FS * sizeof(T)));
         FG_CUDA_TRY(dSlotFace.alloc(S * sizeof(int32_t)));
         FG_CUDA_TRY(dClosure.alloc(3 * (size_t)n * sizeof(T)));
         FG_CUDA_TRY(dFB.alloc((size_t)nF * FREC * sizeof(T)));
-        FG_CUDA_TRY(cudaMemcpy(dFIdx.p, fIdx.data(), 2 * (size_t)nF * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dFGeo.p, fgeo.data(), 11 * FS * sizeof(T), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dSlotFace.p, slotFace.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dClosure.p, closure.data(), 3 * (size_t)n * sizeof(T), cudaMemcpyHostToDevice));
@@ -636,7 +642,7 @@ struct SolverT : public fg_solver {
         const double scal[4] = {cs.dt, 0.0, 0.0, 0.0};
         FG_CUDA_TRY(cudaMemcpy(dScal.p, scal, sizeof(scal), cudaMemcpyHostToDevice));
         bytes = 0;
-        for (DevBuf *b : {&dNbr, &dFlags, &dGeo, &dVol, &dVolP, &dNew2Old, &dU, &dU0, &dRHS, &dStage, &dW[0], &dW[1], &dG,
+        for (DevBuf *b : {&dNbr, &dFlags, &dGeo, &dVol, &dVolP, &dIVol, &dNew2Old, &dU, &dU0, &dRHS, &dStage, &dW[0], &dW[1], &dG,
                           &dSig, &dCellSig, &dBlockMin, &dScal, &dCnt, &dHaloStart, &dHaloIds, &dSlotLocal, &dFIdx, &dFGeo,
                           &dSlotFace, &dClosure, &dFB, &dOrdFlag, &dOrdCnt, &dOrdOff, &dOrder, &dOrdTotal,
                           &dPred, &dHullOk, &dTcErr})
@@ -653,11 +659,10 @@ struct SolverT : public fg_solver {
         dm.aox = g + 0 * GS; dm.aoy = g + 1 * GS; dm.aoz = g + 2 * GS;
         dm.dcx = g + 3 * GS; dm.dcy = g + 4 * GS; dm.dcz = g + 5 * GS;
         dm.vol = dVol.as<double>();
+        dm.ivol = dIVol.as<double>();
         dm.volP = dVolP.as<double>();
         dm.nF = nF;
         dm.fStride = FS;
-        dm.fOwn = dFIdx.as<int32_t>();
-        dm.fNb = dFIdx.as<int32_t>() + nF;
         {
             const T *fg = dFGeo.as<T>();
             dm.fnx = fg; dm.fny = fg + FS; dm.fnz = fg + 2 * FS; dm.fA = fg + 3 * FS;
