@@ -239,24 +239,29 @@ __device__ __forceinline__ void face_state(const T *w, const T *g, T dx, T dy, T
     }
 }
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 // gradient of the liquid-phase temperature T = (p_L + pInf) / (cv (gamma - 1) rho_L) of a cell from
-// its record and gradients (chain rule), added to acc
+// its record and gradients (chain rule), added to acc.  The product is rounded before the sum, so that the
+// sum over a face's two cells does not depend on which comes first (a part of a partitioned mesh may
+// number them the other way round).
 template <typename T>
 __device__ __forceinline__ void cell_grad_t(const PhysT<T> &P, const T *w, const T *g, T *acc) {
     const T rl = w[1], pl = w[6];
     const T c = (pl + P.pinf[0]) / rl;
     const T inv = (T)1 / (P.cvgm1[0] * rl);
 #pragma unroll
-    for (int d = 0; d < 3; d++) acc[d] += (g[NP + 3 * 6 + d] - c * g[NP + 3 * 1 + d]) * inv;
+    for (int d = 0; d < 3; d++) acc[d] += mul_rn(g[NP + 3 * 6 + d] - c * g[NP + 3 * 1 + d], inv);
 }
 
 // Flux part of a face, shared by the face kernels: HLLC + pressure + viscous (+ heat) flux of the
 // reconstructed states sL (owner) and sR (neighbour or ghost), written as the face record of fi.
 // p1: neighbour state for the viscous flux (the cell-centre ghost on a boundary face);
-// gO / gN: the two cells' velocity gradients; gT: sum of their temperature gradients.
+// gs, gT: sums of the two cells' velocity and temperature gradients.
 template <typename T>
-__device__ __forceinline__ T face_tail(const PhysT<T> &P, const T *sL, const T *sR, const T *p1, const T *gO,
-                                          const T *gN, const T *gT, int nb, T nx, T ny, T nz, T A, T lsSq,
+__device__ __forceinline__ T face_tail(const PhysT<T> &P, const T *sL, const T *sR, const T *p1, const T *gs,
+                                          const T *gT, int nb, T nx, T ny, T nz, T A, T lsSq,
                                           int wantSignal, T *__restrict__ FB, size_t nF, int fi) {
     T F[NV], unc, pF;
     hllc_flux(P, sL, sR, nx, ny, nz, F, unc, pF);
@@ -272,7 +277,7 @@ __device__ __forceinline__ T face_tail(const PhysT<T> &P, const T *sL, const T *
     if (P.visc) {
         T gv[9];
 #pragma unroll
-        for (int q = 0; q < 9; q++) gv[q] = (gO[q] + gN[q]) * (T)0.5;
+        for (int q = 0; q < 9; q++) gv[q] = gs[q] * (T)0.5;
         const T nut = P.turb ? wale_nu(gv, lsSq) : (T)0;
         const T dv = (gv[0] + gv[4] + gv[8]) * ((T)2 / 3);
         const T t00 = 2 * gv[0] - dv, t11 = 2 * gv[4] - dv, t22 = 2 * gv[8] - dv;
@@ -334,30 +339,38 @@ __global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(co
                                               T *__restrict__ FB, T *cellSig, const PhysT<T> P, int wantSignal) {
     const int fi = blockIdx.x * blockDim.x + threadIdx.x;
     if (fi >= m.nFEval) return;
-    const int o = m.fOwn[fi];
-    const int nb = m.fNb[fi];
+    const uint32_t lw = m.fLo[fi];
+    const int lo = (int)(lw & 0x7fffffffu), hi = m.fHi[fi];
+    const bool flip = lw >> 31;   // the upper cell is the owner
     const T nx = m.fnx[fi], ny = m.fny[fi], nz = m.fnz[fi], A = m.fA[fi];
-    T wo[NP], sL[NP], sR[NP], p1[NP], gO[9], gN[9];
+    // lanes hold consecutive lower cells, whose records are then consecutive vectors; the upper cells
+    // follow in one direction.  Owner and neighbour are told apart after the reconstruction.
+    T w[NP], sL[NP], sR[NP], p1[NP], gs[9];
     T gT[3] = {0, 0, 0};   // sum of the two cells' temperature gradients (heat conduction)
     {
         T g[GREC];
-        rec_load<T, NP>(W, m.n, o, wo);
-        grec_load<T, GREC>(G, m.n, o, g);
-        face_state(wo, g, m.fdo[0][fi], m.fdo[1][fi], m.fdo[2][fi], sL);
+        rec_load<T, NP>(W, m.n, lo, w);
+        grec_load<T, GREC>(G, m.n, lo, g);
+        face_state(w, g, m.fdl[0][fi], m.fdl[1][fi], m.fdl[2][fi], sL);
 #pragma unroll
-        for (int q = 0; q < 9; q++) gO[q] = g[NP + 9 + q];
-        if (P.heat && nb >= 0) cell_grad_t(P, wo, g, gT);
+        for (int q = 0; q < 9; q++) gs[q] = g[NP + 9 + q];
+        if (P.heat && hi >= 0) cell_grad_t(P, w, g, gT);
     }
-    if (nb >= 0) {
-        T wn[NP], g[GREC];
-        rec_load<T, NP>(W, m.n, nb, wn);
-        grec_load<T, GREC>(G, m.n, nb, g);
-        face_state(wn, g, m.fdn[0][fi], m.fdn[1][fi], m.fdn[2][fi], sR);
+    if (hi >= 0) {
+        T g[GREC];
+        rec_load<T, NP>(W, m.n, hi, w);
+        grec_load<T, GREC>(G, m.n, hi, g);
+        face_state(w, g, m.fdh[0][fi], m.fdh[1][fi], m.fdh[2][fi], sR);
 #pragma unroll
-        for (int q = 0; q < 9; q++) gN[q] = g[NP + 9 + q];
-        if (P.heat) cell_grad_t(P, wn, g, gT);
+        for (int q = 0; q < 9; q++) gs[q] += g[NP + 9 + q];
+        if (P.heat) cell_grad_t(P, w, g, gT);
 #pragma unroll
-        for (int v = 0; v < NP; v++) p1[v] = sR[v];
+        for (int v = 0; v < NP; v++) {
+            const T a = sL[v], b = sR[v];
+            sL[v] = flip ? b : a;
+            sR[v] = flip ? a : b;
+            p1[v] = sR[v];
+        }
     } else {
         // ghost of the reconstructed state for the flux (DP/computeRHS.cu:113); the viscous flux
         // reads the ghost of the cell-centre state (DP/computePrimVec.cu:61-76) and the owner's
@@ -365,18 +378,18 @@ __global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(co
 #pragma unroll
         for (int v = 0; v < NP; v++) {
             sR[v] = sL[v];
-            p1[v] = wo[v];
+            p1[v] = w[v];
         }
-        ghost_state(P, -nb, nx, ny, nz, sR);
-        ghost_state(P, -nb, nx, ny, nz, p1);
+        ghost_state(P, -hi, nx, ny, nz, sR);
+        ghost_state(P, -hi, nx, ny, nz, p1);
 #pragma unroll
-        for (int q = 0; q < 9; q++) gN[q] = gO[q];
+        for (int q = 0; q < 9; q++) gs[q] *= 2;
     }
-    const T sig = face_tail(P, sL, sR, p1, gO, gN, gT, nb, nx, ny, nz, A, m.fLsSq[fi], wantSignal, FB, (size_t)m.nF, fi);
+    const T sig = face_tail(P, sL, sR, p1, gs, gT, hi, nx, ny, nz, A, m.fLsSq[fi], wantSignal, FB, (size_t)m.nF, fi);
     if (wantSignal == 2) {
         // own cells only: a ghost's dt bound belongs to its own part
-        if (o < m.nU) signal_max(cellSig + o, sig);
-        if (nb >= 0 && nb < m.nU) signal_max(cellSig + nb, sig);
+        if (lo < m.nU) signal_max(cellSig + lo, sig);
+        if (hi >= 0 && hi < m.nU) signal_max(cellSig + hi, sig);
     }
 }
 

@@ -33,15 +33,15 @@ struct DevMesh {
     const int32_t *haloStart;
     const int32_t *haloIds;
     const int16_t *slotLocal;
-    // ---- faces (each evaluated once by k_face), in tiles of kFaceTile owner cells: by owner slot,
-    //      then owner cell within a tile ----
+    // ---- faces (each evaluated once by k_face), in tiles of kFaceTile lower cells: by the lower cell's
+    //      slot, then by lower cell within a tile ----
     int nF;
     size_t fStride;                  // component stride of the face geometry arrays
-    const int32_t *fOwn;             // owner cell
-    const int32_t *fNb;              // neighbour cell, or -bc on a boundary face
+    const uint32_t *fLo;             // lower cell (the smaller index); bit 31: the other one is the owner
+    const int32_t *fHi;              // upper cell, or -bc on a boundary face (whose lower cell is the owner)
     const T *fnx, *fny, *fnz, *fA;   // canonical unit normal (owner -> neighbour) and area
-    const T *fdo[3];                 // face centre - owner centre
-    const T *fdn[3];                 // face centre - neighbour centre (periodic image)
+    const T *fdl[3];                 // face centre - lower cell's centre (periodic images as seen from it)
+    const T *fdh[3];                 // face centre - upper cell's centre
     const T *fLsSq;                  // WALE Ls^2 = (0.325 Vavg^0.3333333333333)^2, Vavg = (V_owner +
                                      // V_neighbour) / 2, V_owner on a boundary face
     const int32_t *slotFace;         // [c * nSlots + k] face of a cell slot
@@ -58,9 +58,11 @@ constexpr int FREC = 12;
 #ifndef FG_STAGE_CELLS_D
 #define FG_STAGE_CELLS_D 64
 #endif
-// owner cells per tile of the GPU face order (1: by owner cell, then slot).  Tiles of 32 measured
-// 1-3 % faster per step than 1 on the 128^3 hex workload (the gather reads nearby records) and
-// within 1 % on the graded tet ball.
+// lower cells per tile of the GPU face order: one warp's lanes then hold one local face of 32
+// consecutive cells.  128^3 hexes: face kernel 271 us (291 in tiles of 32 owner cells, whose lanes hold
+// the faces that happen to be owned, half of each direction), gather 194 (201); tiles of 128 lower cells
+// 281 and 203.  FP64 96^3: 325 -> 303 and 125 -> 118 us.  Tets, whose local faces have no common
+// direction: 99 -> 101 us for the face kernel, the gather unchanged.
 #ifndef FG_FACE_TILE
 #define FG_FACE_TILE 32
 #endif

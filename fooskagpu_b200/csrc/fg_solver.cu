@@ -468,49 +468,50 @@ struct SolverT : public fg_solver {
             }
             flags[i] = fl;
         }
-        // faces in GPU order: tiles of kFaceTile consecutive owner cells (renumbered); within a
-        // tile by the owner's element-local face (slot), then by owner.  The lanes of a gather warp
-        // then read the records of the same local face of nearby cells from nearby positions, and
-        // the face kernel's lanes take nearby owners whose neighbours lie in one direction of a hex
-        // brick.  A ghost owns the faces it shares with own cells where the whole mesh makes it the
-        // owner.  On a part the faces touching an own cell come first (the face kernel evaluates
-        // those only); the faces among ghosts, kept for the first-layer ghosts' gradients, follow.
+        // faces in GPU order: tiles of kFaceTile consecutive cells (renumbered); a face belongs to its
+        // lower cell (the smaller index), within a tile by that cell's element-local face (slot), then by
+        // cell.  Along a Morton curve the lower cell of a hex brick's face is the one on its -x / -y / -z
+        // side whatever the element order (and so the owner) is, so the lanes of a warp take one direction
+        // of consecutive cells: the face kernel reads their records as consecutive vectors, and the gather
+        // reads the records of one local face of nearby cells from nearby positions.
+        // On a part the faces touching an own cell come first (the face kernel evaluates those only); the
+        // faces among ghosts, kept for the first-layer ghosts' gradients, follow.
         std::vector<int32_t> gFace(nF, -1), slotFace(S, -1), fIdx(2 * (size_t)nF);
         int nFo = 0;
-        auto touches_own = [&](int f) {
-            return m.old2new[m.fc2el[2 * f]] < nU || (m.boundCond[f] == 0 && m.old2new[m.fc2el[2 * f + 1]] < nU);
-        };
         for (int pass = 0; pass < 2; pass++) {
             for (int t0 = 0; t0 < n; t0 += kFaceTile) {
                 const int t1 = std::min(n, t0 + kFaceTile);
                 for (int k = 0; k < MAXSLOT; k++)
                     for (int i = t0; i < t1; i++) {
-                        const int o = m.new2old[i];
-                        if (k >= fg::elem_type_for_nodes(m.elNN[o])->nFaces) continue;
-                        const int f = elFc2fc[(size_t)o * 6 + k];
-                        if (f >= 0 && elFcSide[(size_t)o * 6 + k] == 0 && touches_own(f) == (pass == 0))
-                            gFace[f] = nFo++;
+                        if (k >= (flags[i] & 7)) continue;
+                        const int c = nbr[(size_t)i * nSlots + k];   // other cell, or -bc
+                        const bool owner = (flags[i] >> (3 + k)) & 1;
+                        if (c >= 0 && (c < i || (c == i && !owner))) continue;
+                        if ((i < nU || (c >= 0 && c < nU)) != (pass == 0)) continue;
+                        const int f = elFc2fc[(size_t)m.new2old[i] * 6 + k];
+                        fIdx[nFo] = (int32_t)((uint32_t)i | (owner ? 0u : 0x80000000u));
+                        fIdx[(size_t)nF + nFo] = c;
+                        gFace[f] = nFo++;
                     }
             }
             if (pass == 0) nFEval = nFo;
         }
-        if (nFo != nF) return set_err(FG_ERR_MESH, "internal: face ownership does not cover every face");
-        // face geometry: 11 components (n[3], A, x_f - x_owner [3], x_f - x_nb [3], WALE Ls^2)
+        if (nFo != nF) return set_err(FG_ERR_MESH, "internal: face order does not cover every face");
+        // face geometry: 11 components (n[3], A, x_f - x_lower [3], x_f - x_upper [3], WALE Ls^2)
         const size_t FS = ((size_t)nF * sizeof(T) + 15) / 16 * 16 / sizeof(T);
         std::vector<T> fgeo(11 * FS, (T)0);
         for (int f = 0; f < nF; f++) {
             const int g = gFace[f];
             const int own = m.fc2el[2 * f], nbo = m.fc2el[2 * f + 1];
             const int bc = m.boundCond[f];
-            fIdx[g] = m.old2new[own];
-            fIdx[(size_t)nF + g] = (bc == 0) ? m.old2new[nbo] : -bc;
             for (int d = 0; d < 3; d++) fgeo[(size_t)d * FS + g] = (T)m.n[(size_t)f * 3 + d];
             fgeo[3 * FS + g] = (T)m.area[f];
+            const int cO = fIdx[g] < 0 ? 7 : 4;   // the owner's components: it is the upper / the lower cell
             for (int d = 0; d < 3; d++) {
                 const double xf = m.fcCenter[(size_t)f * 3 + d];
-                fgeo[(size_t)(4 + d) * FS + g] = (T)(xf - m.cellCenter[(size_t)own * 3 + d]);
+                fgeo[(size_t)(cO + d) * FS + g] = (T)(xf - m.cellCenter[(size_t)own * 3 + d]);
                 if (bc == 0)
-                    fgeo[(size_t)(7 + d) * FS + g] =
+                    fgeo[(size_t)(11 - cO + d) * FS + g] =
                         (T)((xf + m.nbShift[(size_t)f * 3 + d]) - m.cellCenter[(size_t)nbo * 3 + d]);
             }
             // WALE length scale squared of the face (DP/computeViscousStresses.cu:54-56)
@@ -600,8 +601,8 @@ struct SolverT : public fg_solver {
         FG_CUDA_TRY(cudaMemcpy(dNew2Old.p, m.new2old.data(), (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(dFIdx.alloc(2 * (size_t)nF * sizeof(int32_t)));
         FG_CUDA_TRY(cudaMemcpy(dFIdx.p, fIdx.data(), 2 * (size_t)nF * sizeof(int32_t), cudaMemcpyHostToDevice));
-        dm.fOwn = dFIdx.as<int32_t>();
-        dm.fNb = dFIdx.as<int32_t>() + nF;
+        dm.fLo = dFIdx.as<uint32_t>();
+        dm.fHi = dFIdx.as<int32_t>() + nF;
         FG_CUDA_TRY(dFGeo.alloc(11 * FS * sizeof(T)));
         FG_CUDA_TRY(dSlotFace.alloc(S * sizeof(int32_t)));
         FG_CUDA_TRY(dClosure.alloc(3 * (size_t)n * sizeof(T)));
@@ -667,8 +668,8 @@ struct SolverT : public fg_solver {
             const T *fg = dFGeo.as<T>();
             dm.fnx = fg; dm.fny = fg + FS; dm.fnz = fg + 2 * FS; dm.fA = fg + 3 * FS;
             for (int d = 0; d < 3; d++) {
-                dm.fdo[d] = fg + (4 + d) * FS;
-                dm.fdn[d] = fg + (7 + d) * FS;
+                dm.fdl[d] = fg + (4 + d) * FS;
+                dm.fdh[d] = fg + (7 + d) * FS;
             }
             dm.fLsSq = fg + 10 * FS;
         }
