@@ -15,9 +15,10 @@
 
 namespace fg {
 
-// Primitive record: [alpha, rhoL, rhoG, u, v, w, pL, pG, m_v]; stored padded to WREC.
+// Primitive record: [alpha, rhoL, rhoG, u, v, w, pL, pG, m_v], WREC values allocated per cell.
 constexpr int NP = 9;
 constexpr int WREC = 12;
+constexpr int WVEC = 8;   // values in 16-byte vectors; the others in planes of single values
 // Per-cell limited-gradient record: theta[9] then grad[9][3].
 constexpr int GREC = 36;
 constexpr int NV = 10;
@@ -70,6 +71,26 @@ __device__ __forceinline__ void rec_store(T *base, size_t stride, int c, const T
         else x = make_double2(val(2 * q), val(2 * q + 1));
         b[(size_t)q * stride + c] = x;
     }
+}
+
+// The primitive records W: values 0 .. WVEC - 1 as above, value v >= WVEC of cell c at base[v * stride + c].
+// The ninth value (the vapour mass) then costs 4 (8) bytes and one cache line per warp where a vector
+// of its own, three quarters (one half) padding, cost 16 and four.
+template <typename T>
+__host__ __device__ inline size_t w_index(size_t stride, size_t c, int v) {
+    return v < WVEC ? rec_index<T>(stride, c, v) : (size_t)v * stride + c;
+}
+template <typename T>
+__device__ __forceinline__ void w_load(const T *__restrict__ base, size_t stride, int c, T *out) {
+    rec_load<T, WVEC>(base, stride, c, out);
+#pragma unroll
+    for (int v = WVEC; v < NP; v++) out[v] = __ldg(base + (size_t)v * stride + c);
+}
+template <typename T>
+__device__ __forceinline__ void w_store(T *base, size_t stride, int c, const T *in) {
+    rec_store<T, WVEC>(base, stride, c, in);
+#pragma unroll
+    for (int v = WVEC; v < NP; v++) base[(size_t)v * stride + c] = in[v];
 }
 
 // The gradient records G use the same component-major layout with vectors of 16 or 32 bytes per

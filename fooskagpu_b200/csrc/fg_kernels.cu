@@ -62,21 +62,30 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *g) {
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <typename T>
-__host__ __device__ constexpr int stage_w_vecs() { return (NP + vpv<T>() - 1) / vpv<T>(); }
-template <typename T>
-constexpr size_t grad_smem(int rows) { return (size_t)rows * stage_w_vecs<T>() * 16; }
+__device__ __forceinline__ void cp_async_value(T *smem, const T *g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g),
+                 "n"(sizeof(T))
+                 : "memory");
+}
 
-// NVAL values of staged record r from the planes of 16-byte vectors starting at plane q0
-template <typename T, int NVAL>
-__device__ __forceinline__ void staged_load(const typename Vec16<T>::type *sm, int rows, int q0, int r, T *out) {
-    constexpr int P = vpv<T>();
+template <typename T>
+__host__ __device__ constexpr int stage_w_vecs() { return WVEC / vpv<T>(); }
+template <typename T>
+constexpr size_t grad_smem(int rows) { return (size_t)rows * (stage_w_vecs<T>() * 16 + (NP - WVEC) * sizeof(T)); }
+
+// staged primitive record r: the planes of vectors, then the single values
+template <typename T>
+__device__ __forceinline__ void staged_load(const typename Vec16<T>::type *sm, int rows, int r, T *out) {
+    constexpr int P = vpv<T>(), Q = stage_w_vecs<T>();
 #pragma unroll
-    for (int q = 0; q < (NVAL + P - 1) / P; q++) {
-        const typename Vec16<T>::type x = sm[(q0 + q) * rows + r];
+    for (int q = 0; q < Q; q++) {
+        const typename Vec16<T>::type x = sm[q * rows + r];
 #pragma unroll
-        for (int j = 0; j < P; j++)
-            if (q * P + j < NVAL) out[q * P + j] = vlane(x, j);
+        for (int j = 0; j < P; j++) out[q * P + j] = vlane(x, j);
     }
+    const T *tail = reinterpret_cast<const T *>(sm + Q * rows);
+#pragma unroll
+    for (int v = WVEC; v < NP; v++) out[v] = tail[(v - WVEC) * rows + r];
 }
 
 // two consecutive values of a per-slot array
@@ -126,18 +135,35 @@ __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_gr
         const int src = r < B ? lo + r : m.haloIds[hs + r - B];
 #pragma unroll
         for (int q = 0; q < WQ; q++) cp_async16(sm + q * rows + r, reinterpret_cast<const V *>(W) + (size_t)q * m.n + src);
+#pragma unroll
+        for (int v = WVEC; v < NP; v++)
+            cp_async_value(reinterpret_cast<T *>(sm + WQ * rows) + (v - WVEC) * rows + r, W + (size_t)v * m.n + src);
     }
     const int t = threadIdx.x;
     const int c = lo + t;
     const bool own = t < nOwn;
     const int fl = own ? m.flags[c] : 0;
     const T iv = own ? (T)m.ivol[c] : (T)0;
+    // the geometry of the first PRE slots is in flight together with the records.  128^3 hexes, FP32: 6 slots
+    // 170 us, 2 slots 172, none 175; FP64 96^3 (registers are short there): 2 slots 205, 4 slots 209, none 212
+    constexpr int PRE = sizeof(T) == 4 ? 6 : 2;
+    const size_t g0 = (size_t)c * S;
+    T ax[S], ay[S], az[S];
+    int sl[S / 2];
+    if (own) {
+#pragma unroll
+        for (int k2 = 0; k2 < PRE && k2 < S; k2 += 2) {
+            load_pair(m.aox + g0 + k2, ax + k2);
+            load_pair(m.aoy + g0 + k2, ay + k2);
+            load_pair(m.aoz + g0 + k2, az + k2);
+            sl[k2 / 2] = __ldg(reinterpret_cast<const int *>(m.slotLocal + g0 + k2));
+        }
+    }
     cp_async_wait();
     __syncthreads();
     if (!own) return;
-    const size_t g0 = (size_t)c * S;
     T w[NP], gs[NP * 3], mn[NP], mx[NP];
-    staged_load<T, NP>(sm, rows, 0, t, w);
+    staged_load<T>(sm, rows, t, w);
 #pragma unroll
     for (int v = 0; v < NP; v++) {
         gs[3 * v] = gs[3 * v + 1] = gs[3 * v + 2] = 0;
@@ -148,23 +174,24 @@ __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_gr
 #pragma unroll
     for (int k2 = 0; k2 < S; k2 += 2) {
         if (k2 >= nf) break;
-        T ax[2], ay[2], az[2];
-        load_pair(m.aox + g0 + k2, ax);
-        load_pair(m.aoy + g0 + k2, ay);
-        load_pair(m.aoz + g0 + k2, az);
-        const int sl = __ldg(reinterpret_cast<const int *>(m.slotLocal + g0 + k2));
+        if (k2 >= PRE) {
+            load_pair(m.aox + g0 + k2, ax + k2);
+            load_pair(m.aoy + g0 + k2, ay + k2);
+            load_pair(m.aoz + g0 + k2, az + k2);
+            sl[k2 / 2] = __ldg(reinterpret_cast<const int *>(m.slotLocal + g0 + k2));
+        }
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             const int k = k2 + j;
             if (k >= nf) break;
-            const int li = j ? sl >> 16 : (int)(int16_t)sl;
+            const int li = j ? sl[k2 / 2] >> 16 : (int)(int16_t)sl[k2 / 2];
             // half the outward n A of the face (the host computed (+-1) n A in T arithmetic, as the
             // reference's sign times normal times area): (w + w_nb) times it is exactly the mean
             // times the whole
-            const T hx = ax[j] * (T)0.5, hy = ay[j] * (T)0.5, hz = az[j] * (T)0.5;
+            const T hx = ax[k] * (T)0.5, hy = ay[k] * (T)0.5, hz = az[k] * (T)0.5;
             T ot[NP];
             if (li >= 0) {
-                staged_load<T, NP>(sm, rows, 0, li, ot);
+                staged_load<T>(sm, rows, li, ot);
             } else {
                 // boundary slot: the cell owns the face, so its canonical normal points outward
                 const int fi = m.slotFace[g0 + k];
@@ -349,7 +376,7 @@ __global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(co
     T gT[3] = {0, 0, 0};   // sum of the two cells' temperature gradients (heat conduction)
     {
         T g[GREC];
-        rec_load<T, NP>(W, m.n, lo, w);
+        w_load<T>(W, m.n, lo, w);
         grec_load<T, GREC>(G, m.n, lo, g);
         face_state(w, g, m.fdl[0][fi], m.fdl[1][fi], m.fdl[2][fi], sL);
 #pragma unroll
@@ -358,7 +385,7 @@ __global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(co
     }
     if (hi >= 0) {
         T g[GREC];
-        rec_load<T, NP>(W, m.n, hi, w);
+        w_load<T>(W, m.n, hi, w);
         grec_load<T, GREC>(G, m.n, hi, g);
         face_state(w, g, m.fdh[0][fi], m.fdh[1][fi], m.fdh[2][fi], sR);
 #pragma unroll
@@ -443,8 +470,8 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
             su += s * (double)rec[NV];
             sig = fmax(sig, rec[NV + 1]);
         }
-        T w[NP];
-        rec_load<T, NP>(f.Win, m.n, c, w);
+        T w[WVEC];
+        rec_load<T, WVEC>(f.Win, m.n, c, w);
         const double a = w[0], pl = w[6], pg = w[7];
         const double pc = (double)(w[0] * w[6] + (1 - w[0]) * w[7]) - D.pDatum;
         acc[0] -= a * su;
@@ -488,7 +515,7 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
             if (!state_ok(u)) *f.bad = f.step + 1;
             T wo[NP];
             cons2prim_d(D, u, wo);
-            rec_store<T, NP>(f.Wout, m.n, c, wo);
+            w_store<T>(f.Wout, m.n, c, wo);
         }
     }
     if (wantSignal) {
@@ -557,7 +584,7 @@ __global__ void k_update(const DevMesh<T> m, Fields<T> f, const PhysD D, StageCo
     if (!state_ok(u)) *f.bad = f.step + 1;
     T wo[NP];
     cons2prim_d(D, u, wo);
-    rec_store<T, NP>(f.Wout, m.n, c, wo);
+    w_store<T>(f.Wout, m.n, c, wo);
 }
 
 template <typename T>
@@ -569,7 +596,7 @@ __global__ void k_prim(int n, const double *__restrict__ U, T *W, size_t wStride
     for (int v = 0; v < NV; v++) u[v] = U[(size_t)v * n + c];
     T w[NP];
     cons2prim_d(D, u, w);
-    rec_store<T, NP>(W, wStride, c, w);
+    w_store<T>(W, wStride, c, w);
 }
 
 __global__ void k_dt_finalize(const double *blockMin, int nb, double cfl, double maxDt, double *dt) {
@@ -721,12 +748,26 @@ __global__ void k_scatter_state(int n, const double *__restrict__ Ua, const int3
 #pragma unroll
     for (int v = 0; v < NV; v++) U[(size_t)v * n + c] = Ua[o + v];
 }
-__global__ void k_gather_state(int n, const double *__restrict__ U, const int32_t *__restrict__ new2old, double *Ua) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const size_t o = (size_t)new2old[c] * NV;
+// the state in the caller's order and layout: a block collects kStateCells cells in shared memory and
+// writes each cell's 80 bytes with 5 consecutive lanes (scattered 8-byte stores of one lane per cell
+// took 264 us for 2.1 M cells)
+constexpr int kStateCells = 128;
+__global__ void __launch_bounds__(kStateCells) k_gather_state(int n, const double *__restrict__ U,
+                                                              const int32_t *__restrict__ new2old, double *__restrict__ Ua) {
+    __shared__ double2 sh[kStateCells][NV / 2];
+    __shared__ int32_t to[kStateCells];
+    const int lo = blockIdx.x * kStateCells, c = lo + threadIdx.x, cnt = min(kStateCells, n - lo);
+    if (c < n) {
+        to[threadIdx.x] = new2old[c];
 #pragma unroll
-    for (int v = 0; v < NV; v++) Ua[o + v] = U[(size_t)v * n + c];
+        for (int v = 0; v < NV; v += 2)
+            sh[threadIdx.x][v / 2] = make_double2(U[(size_t)v * n + c], U[(size_t)(v + 1) * n + c]);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < cnt * (NV / 2); q += kStateCells) {
+        const int r = q / (NV / 2), v = q - r * (NV / 2);
+        reinterpret_cast<double2 *>(Ua)[(size_t)to[r] * (NV / 2) + v] = sh[r][v];
+    }
 }
 __global__ void k_copy(size_t cnt, const double *__restrict__ a, double *b) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -735,26 +776,26 @@ __global__ void k_copy(size_t cnt, const double *__restrict__ a, double *b) {
 }
 
 // ------------------------------------------------------------------ halo records (partitioned runs)
-// out[k * nval + v] = value v of the record of cells[k] (records of nRec cells, nval values each):
+// out[k * nval + v] = value v of the primitive record of cells[k] (records of nRec cells, nval values each):
 // the records of the cells another part needs, packed whole
 template <typename T>
-__global__ void k_halo_pack(const T *__restrict__ rec, size_t nRec, int nval, int vpv, const int32_t *__restrict__ cells,
+__global__ void k_halo_pack(const T *__restrict__ rec, size_t nRec, int nval, const int32_t *__restrict__ cells,
                             int cnt, T *__restrict__ out) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)cnt * nval) return;
     const size_t k = i / nval;
     const int v = (int)(i - k * nval);
-    out[i] = rec[((size_t)(v / vpv) * nRec + (size_t)cells[k]) * vpv + (size_t)(v % vpv)];
+    out[i] = rec[w_index<T>(nRec, (size_t)cells[k], v)];
 }
 // value v of the record of cells[k] = in[k * nval + v]: the ghosts' records received from their parts
 template <typename T>
-__global__ void k_halo_unpack(T *__restrict__ rec, size_t nRec, int nval, int vpv, const int32_t *__restrict__ cells,
+__global__ void k_halo_unpack(T *__restrict__ rec, size_t nRec, int nval, const int32_t *__restrict__ cells,
                               int cnt, const T *__restrict__ in) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)cnt * nval) return;
     const size_t k = i / nval;
     const int v = (int)(i - k * nval);
-    rec[((size_t)(v / vpv) * nRec + (size_t)cells[k]) * vpv + (size_t)(v % vpv)] = in[i];
+    rec[w_index<T>(nRec, (size_t)cells[k], v)] = in[i];
 }
 
 // ------------------------------------------------------------------ launchers
@@ -807,21 +848,21 @@ void launch_update(const DevMesh<T> &m, const Fields<T> &f, const PhysD &D, Stag
     k_update<T><<<(m.nU + 255) / 256, 256, 0, s>>>(m, f, D, sc);
 }
 template <typename T>
-void launch_halo_pack(const T *rec, size_t nRec, int nval, int vpv, const int32_t *cells, int cnt, T *out,
+void launch_halo_pack(const T *rec, size_t nRec, int nval, const int32_t *cells, int cnt, T *out,
                       cudaStream_t s) {
     const size_t tot = (size_t)cnt * nval;
-    if (tot) k_halo_pack<T><<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(rec, nRec, nval, vpv, cells, cnt, out);
+    if (tot) k_halo_pack<T><<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(rec, nRec, nval, cells, cnt, out);
 }
 template <typename T>
-void launch_halo_unpack(T *rec, size_t nRec, int nval, int vpv, const int32_t *cells, int cnt, const T *in,
+void launch_halo_unpack(T *rec, size_t nRec, int nval, const int32_t *cells, int cnt, const T *in,
                         cudaStream_t s) {
     const size_t tot = (size_t)cnt * nval;
-    if (tot) k_halo_unpack<T><<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(rec, nRec, nval, vpv, cells, cnt, in);
+    if (tot) k_halo_unpack<T><<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(rec, nRec, nval, cells, cnt, in);
 }
-template void launch_halo_pack<float>(const float *, size_t, int, int, const int32_t *, int, float *, cudaStream_t);
-template void launch_halo_pack<double>(const double *, size_t, int, int, const int32_t *, int, double *, cudaStream_t);
-template void launch_halo_unpack<float>(float *, size_t, int, int, const int32_t *, int, const float *, cudaStream_t);
-template void launch_halo_unpack<double>(double *, size_t, int, int, const int32_t *, int, const double *, cudaStream_t);
+template void launch_halo_pack<float>(const float *, size_t, int, const int32_t *, int, float *, cudaStream_t);
+template void launch_halo_pack<double>(const double *, size_t, int, const int32_t *, int, double *, cudaStream_t);
+template void launch_halo_unpack<float>(float *, size_t, int, const int32_t *, int, const float *, cudaStream_t);
+template void launch_halo_unpack<double>(double *, size_t, int, const int32_t *, int, const double *, cudaStream_t);
 template <typename T>
 void launch_prim(int n, const double *U, T *W, size_t wStride, const PhysD &D, cudaStream_t s) {
     k_prim<T><<<(n + 255) / 256, 256, 0, s>>>(n, U, W, wStride, D);
@@ -850,7 +891,7 @@ void launch_scatter_state(int n, const double *Ua, const int32_t *new2old, doubl
     k_scatter_state<<<(n + 255) / 256, 256, 0, s>>>(n, Ua, new2old, U, firstBad, flags);
 }
 void launch_gather_state(int n, const double *U, const int32_t *new2old, double *Ua, cudaStream_t s) {
-    k_gather_state<<<(n + 255) / 256, 256, 0, s>>>(n, U, new2old, Ua);
+    k_gather_state<<<(n + kStateCells - 1) / kStateCells, kStateCells, 0, s>>>(n, U, new2old, Ua);
 }
 void launch_copy_u0(int n, const double *U, double *U0, cudaStream_t s) {
     const size_t cnt = (size_t)n * NV;

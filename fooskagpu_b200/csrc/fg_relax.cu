@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
                 U[(size_t)9 * n + c] = u[9];
                 T w[NP];
                 cons2prim_d(D, u, w);
-                rec_store<T, NP>(W, wStride, c, w);
+                w_store<T>(W, wStride, c, w);
                 hullOk[i] = kPolished;
             }
         }
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINB
         U[(size_t)9 * n + c] = u[9];
         T w[NP];
         cons2prim_d(D, u, w);
-        rec_store<T, NP>(W, wStride, c, w);
+        w_store<T>(W, wStride, c, w);
     }
     // warp-aggregated counters (sums of integers: order does not matter)
     const unsigned mask = __ballot_sync(0xffffffffu, act && chem);

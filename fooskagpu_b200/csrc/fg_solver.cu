@@ -810,17 +810,16 @@ struct SolverT : public fg_solver {
         if (field != FG_HALO_W) return set_err(FG_ERR_ARG, "partitioned run: only primitive records are exchanged");
         T *rec = dW[cur].as<T>();
         const int stride = WREC;
-        const int vpvRec = vpv<T>();
         const int nSend = sendStart.back(), nRecv = recvStart.back();
         prof_begin(FG_K_OTHER, s);
-        launch_halo_pack<T>(rec, (size_t)n, stride, vpvRec, dSendCells.as<int32_t>(), nSend, static_cast<T *>(haloSend), s);
+        launch_halo_pack<T>(rec, (size_t)n, stride, dSendCells.as<int32_t>(), nSend, static_cast<T *>(haloSend), s);
         prof_end(s);
         FG_LAUNCH_CHECK("halo pack");
         FG_CUDA_TRY(cudaStreamSynchronize(s));
         if (halo.exchange(halo.ctx, field, (int64_t)stride * (int64_t)sizeof(T), s) != 0)
             return set_err(FG_ERR_CUDA, "partitioned run: halo exchange failed");
         prof_begin(FG_K_OTHER, s);
-        launch_halo_unpack<T>(rec, (size_t)n, stride, vpvRec, dRecvCells.as<int32_t>(), nRecv,
+        launch_halo_unpack<T>(rec, (size_t)n, stride, dRecvCells.as<int32_t>(), nRecv,
                             static_cast<const T *>(haloRecv), s);
         prof_end(s);
         FG_LAUNCH_CHECK("halo unpack");
