@@ -45,13 +45,13 @@ __device__ __forceinline__ float vlane(const float4 &x, int j) { return j == 0 ?
 __device__ __forceinline__ double vlane(const double2 &x, int j) { return j == 0 ? x.x : x.y; }
 // the first NVAL values of the record of cell c
 template <typename T, int NVAL>
-__device__ __forceinline__ void rec_load(const T *__restrict__ base, size_t stride, int c, T *out) {
+__device__ __forceinline__ void rec_load(const T *base, size_t stride, int c, T *out) {
     using V = typename Vec16<T>::type;
     constexpr int P = vpv<T>();
     const V *b = reinterpret_cast<const V *>(base);
 #pragma unroll
     for (int q = 0; q < (NVAL + P - 1) / P; q++) {
-        const V x = __ldg(b + (size_t)q * stride + c);
+        const V x = b[(size_t)q * stride + c];
 #pragma unroll
         for (int j = 0; j < P; j++)
             if (q * P + j < NVAL) out[q * P + j] = vlane(x, j);
@@ -81,10 +81,10 @@ __host__ __device__ inline size_t w_index(size_t stride, size_t c, int v) {
     return v < WVEC ? rec_index<T>(stride, c, v) : (size_t)v * stride + c;
 }
 template <typename T>
-__device__ __forceinline__ void w_load(const T *__restrict__ base, size_t stride, int c, T *out) {
+__device__ __forceinline__ void w_load(const T *base, size_t stride, int c, T *out) {
     rec_load<T, WVEC>(base, stride, c, out);
 #pragma unroll
-    for (int v = WVEC; v < NP; v++) out[v] = __ldg(base + (size_t)v * stride + c);
+    for (int v = WVEC; v < NP; v++) out[v] = base[(size_t)v * stride + c];
 }
 template <typename T>
 __device__ __forceinline__ void w_store(T *base, size_t stride, int c, const T *in) {
@@ -114,15 +114,14 @@ template <typename T>
 __host__ __device__ inline size_t grec_index(size_t stride, size_t c, int v) {
     return ((size_t)(v / gvec<T>()) * stride + c) * gvec<T>() + (size_t)(v % gvec<T>());
 }
-// one 32-byte vector: the loads read data that is not written during the kernel (non-coherent
-// path), the stores are ordinary
+// one 32-byte vector (volatile: not moved before the wait for the kernel that wrote it, see pdl_wait)
 __device__ __forceinline__ void ld32(const float *p, float *r) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
         : "l"(p));
 }
 __device__ __forceinline__ void ld32(const double *p, double *r) {
-    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3]) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3]) : "l"(p));
 }
 __device__ __forceinline__ void st32(float *p, const float *r) {
     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(r[0]), "f"(r[1]), "f"(r[2]),
@@ -135,7 +134,7 @@ __device__ __forceinline__ void st32(double *p, const double *r) {
 }
 // the first NVAL values of the G record of cell c
 template <typename T, int NVAL>
-__device__ __forceinline__ void grec_load(const T *__restrict__ base, size_t stride, int c, T *out) {
+__device__ __forceinline__ void grec_load(const T *base, size_t stride, int c, T *out) {
     if constexpr (gvec_bytes<T>() == 16) {
         rec_load<T, NVAL>(base, stride, c, out);
     } else {

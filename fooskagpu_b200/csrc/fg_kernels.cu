@@ -38,12 +38,12 @@ __device__ __forceinline__ void store_frec(T *FB, size_t nF, int f, const T *r) 
     }
 }
 template <typename T>
-__device__ __forceinline__ void load_frec(const T *__restrict__ FB, size_t nF, int f, T *r) {
+__device__ __forceinline__ void load_frec(const T *FB, size_t nF, int f, T *r) {
     if constexpr (sizeof(T) == 8) {
         rec_load<T, FREC>(FB, nF, f, r);
     } else {
         const float4 *p = reinterpret_cast<const float4 *>(FB + (size_t)f * FREC);
-        const float4 a = __ldg(p), b = __ldg(p + 1), d = __ldg(p + 2);
+        const float4 a = p[0], b = p[1], d = p[2];
         r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
         r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
         r[8] = d.x; r[9] = d.y; r[10] = d.z; r[11] = d.w;
@@ -118,8 +118,8 @@ __device__ __forceinline__ T limiter_phi(T num, T diff) {
 // Measured against scalar loads and records staged value by value: FP32 196 -> 177 us (128^3 hexes),
 // 86 -> 78 (981 k tets); FP64 224 -> 213 (96^3 hexes), 123 -> 109 (480 k tets).
 template <typename T, int kLim, int S>
-__global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_grad(const DevMesh<T> m, const T *__restrict__ W,
-                                                                T *__restrict__ G, const PhysT<T> P) {
+__global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_grad(const DevMesh<T> m, const T *W,
+                                                                T *G, const PhysT<T> P) {
     using V = typename Vec16<T>::type;
     constexpr int B = StageCells<T>::value, WQ = stage_w_vecs<T>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -129,16 +129,9 @@ __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_gr
     const int nOwn = min(B, m.nG - lo);       // cells whose gradients this block computes
     const int nBlockRecs = min(B, m.n - lo);  // cells of the block range with records (ghosts of a part too)
     const int rows = B + m.maxHalo;
+    pdl_trigger();
     const int hs = m.haloStart[b], nRec = B + (m.haloStart[b + 1] - hs);
-    for (int r = threadIdx.x; r < nRec; r += B) {
-        if (r < B && r >= nBlockRecs) continue;
-        const int src = r < B ? lo + r : m.haloIds[hs + r - B];
-#pragma unroll
-        for (int q = 0; q < WQ; q++) cp_async16(sm + q * rows + r, reinterpret_cast<const V *>(W) + (size_t)q * m.n + src);
-#pragma unroll
-        for (int v = WVEC; v < NP; v++)
-            cp_async_value(reinterpret_cast<T *>(sm + WQ * rows) + (v - WVEC) * rows + r, W + (size_t)v * m.n + src);
-    }
+    const int id1 = threadIdx.x + B < nRec ? m.haloIds[hs + threadIdx.x] : 0;
     const int t = threadIdx.x;
     const int c = lo + t;
     const bool own = t < nOwn;
@@ -158,6 +151,16 @@ __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_gr
             load_pair(m.aoz + g0 + k2, az + k2);
             sl[k2 / 2] = __ldg(reinterpret_cast<const int *>(m.slotLocal + g0 + k2));
         }
+    }
+    pdl_wait();
+    for (int r = threadIdx.x; r < nRec; r += B) {
+        if (r < B && r >= nBlockRecs) continue;
+        const int src = r < B ? lo + r : (r < 2 * B ? id1 : m.haloIds[hs + r - B]);
+#pragma unroll
+        for (int q = 0; q < WQ; q++) cp_async16(sm + q * rows + r, reinterpret_cast<const V *>(W) + (size_t)q * m.n + src);
+#pragma unroll
+        for (int v = WVEC; v < NP; v++)
+            cp_async_value(reinterpret_cast<T *>(sm + WQ * rows) + (v - WVEC) * rows + r, W + (size_t)v * m.n + src);
     }
     cp_async_wait();
     __syncthreads();
@@ -362,13 +365,16 @@ __device__ __forceinline__ void signal_max(double *a, double v) {
 //   var 0: -alpha_c s u,  vars 6/7: +alpha_c pL_c s u, +(1-alpha_c) pG_c s u,
 //   momentum: -pC_c s A n summed = pC_c * (sum of outward n A)  (DP/flux.h:1-30, DP/computeRHS.cu:38-75)
 template <typename T>
-__global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(const DevMesh<T> m, const T *__restrict__ W, const T *__restrict__ G,
-                                              T *__restrict__ FB, T *cellSig, const PhysT<T> P, int wantSignal) {
+__global__ void __launch_bounds__(FG_FACE_THREADS, MinBlocks<T>::face) k_face(const DevMesh<T> m, const T *W, const T *G,
+                                              T *FB, T *cellSig, const PhysT<T> P, int wantSignal) {
     const int fi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (fi >= m.nFEval) return;
-    const uint32_t lw = m.fLo[fi];
-    const int lo = (int)(lw & 0x7fffffffu), hi = m.fHi[fi];
+    const bool on = fi < m.nFEval;
+    pdl_trigger();
+    const uint32_t lw = on ? m.fLo[fi] : 0;
+    const int lo = (int)(lw & 0x7fffffffu), hi = on ? m.fHi[fi] : 0;
     const bool flip = lw >> 31;   // the upper cell is the owner
+    pdl_wait();
+    if (!on) return;
     const T nx = m.fnx[fi], ny = m.fny[fi], nz = m.fnz[fi], A = m.fA[fi];
     // lanes hold consecutive lower cells, whose records are then consecutive vectors; the upper cells
     // follow in one direction.  Owner and neighbour are told apart after the reconstruction.
@@ -449,15 +455,19 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = m.nU;   // state rows (U, U0, RHS stride)
     double cfl = 1e12;
+    pdl_trigger();
+    int id[S], fl = 0;
     if (c < n) {
-        const int fl = m.flags[c];
+        fl = m.flags[c];
+        load_slot_faces<S>(m.slotFace + (size_t)c * S, id);
+    }
+    pdl_wait();
+    if (c < n) {
         const int nf = fl & 7;
         double acc[NV], su = 0.0;
 #pragma unroll
         for (int v = 0; v < NV; v++) acc[v] = 0.0;
         T sig = (T)-1e9;
-        int id[S];
-        load_slot_faces<S>(m.slotFace + (size_t)c * S, id);
 #pragma unroll
         for (int k = 0; k < S; k++) {
             if (k >= nf) break;
@@ -537,7 +547,9 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
 // the gather kernel computes it on the residual path: signal[c], then the deterministic block
 // minimum of volP / signal over blocks of the gather kernel's size
 template <typename T>
-__global__ void k_cell_cfl(const DevMesh<T> m, const T *__restrict__ cellSig, double *signal, double *blockMin) {
+__global__ void k_cell_cfl(const DevMesh<T> m, const T *cellSig, double *signal, double *blockMin) {
+    pdl_trigger();
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double cfl = 1e12;
     if (c < m.nU) {
@@ -560,6 +572,8 @@ __global__ void k_cell_cfl(const DevMesh<T> m, const T *__restrict__ cellSig, do
 // RK stage from the RHS buffer (DP/update.cu:19-103)
 template <typename T>
 __global__ void k_update(const DevMesh<T> m, Fields<T> f, const PhysD D, StageCoef sc) {
+    pdl_trigger();
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = m.nU;
     if (c >= n) return;
@@ -600,6 +614,8 @@ __global__ void k_prim(int n, const double *__restrict__ U, T *W, size_t wStride
 }
 
 __global__ void k_dt_finalize(const double *blockMin, int nb, double cfl, double maxDt, double *dt) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ double red[32];
     double v = 1e12;
     for (int i = threadIdx.x; i < nb; i += blockDim.x) v = fmin(v, blockMin[i]);
@@ -616,8 +632,10 @@ __global__ void k_dt_finalize(const double *blockMin, int nb, double cfl, double
 
 // ------------------------------------------------------------------ conservation (DP/consCalc.cu:3-34)
 constexpr int kConsThreads = 256;
-__global__ void k_cons_blocks(int n, int ivar, const double *__restrict__ U, const double *__restrict__ vol,
+__global__ void k_cons_blocks(int n, int ivar, const double *U, const double *__restrict__ vol,
                               double *blockSum) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ double sh[kConsThreads];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.0;
@@ -634,6 +652,8 @@ __global__ void k_cons_blocks(int n, int ivar, const double *__restrict__ U, con
     if (threadIdx.x == 0) blockSum[blockIdx.x] = sh[0];
 }
 __global__ void k_cons_final(const double *blockSum, int nb, double *out) {
+    pdl_trigger();
+    pdl_wait();
     // fixed-shape tree over per-thread strided partial sums: deterministic for a given nb
     __shared__ double sh[1024];
     double v = 0.0;
@@ -823,29 +843,29 @@ void launch_grad(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, cud
     const size_t sm = grad_smem<T>(m.blockCells + m.maxHalo);
     auto *k = m.nSlots == 4 ? (P.limiter == 1 ? k_grad<T, 1, 4> : k_grad<T, 0, 4>)
                             : (P.limiter == 1 ? k_grad<T, 1, 6> : k_grad<T, 0, 6>);
-    k<<<nb, m.blockCells, sm, s>>>(m, f.Win, f.G, P);
+    launch_pdl(k, nb, m.blockCells, sm, s, m, f.Win, f.G, P);
 }
 template <typename T>
 void launch_face(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, int wantSignal, cudaStream_t s) {
     if (m.nFEval == 0) return;
-    k_face<T><<<(m.nFEval + FG_FACE_THREADS - 1) / FG_FACE_THREADS, FG_FACE_THREADS, 0, s>>>(m, f.Win, f.G, f.FB, f.cellSig, P,
-                                                                                      wantSignal);
+    launch_pdl(k_face<T>, (m.nFEval + FG_FACE_THREADS - 1) / FG_FACE_THREADS, FG_FACE_THREADS, 0, s, m, f.Win, f.G, f.FB,
+               f.cellSig, P, wantSignal);
 }
 template <typename T>
 void launch_cell_cfl(const DevMesh<T> &m, const Fields<T> &f, cudaStream_t s) {
-    k_cell_cfl<T><<<flux_blocks(m.nU), kGatherThreads, 0, s>>>(m, f.cellSig, f.signal, f.blockMin);
+    launch_pdl(k_cell_cfl<T>, flux_blocks(m.nU), kGatherThreads, 0, s, m, f.cellSig, f.signal, f.blockMin);
 }
 template <typename T>
 void launch_gather(const DevMesh<T> &m, const Fields<T> &f, const PhysD &D, int mode, int wantSignal,
                    StageCoef sc, cudaStream_t s) {
     auto *k = m.nSlots == 4 ? k_gather<T, 4> : k_gather<T, 6>;
-    k<<<flux_blocks(m.nU), kGatherThreads, 0, s>>>(m, f, D, mode, wantSignal, sc);
+    launch_pdl(k, flux_blocks(m.nU), kGatherThreads, 0, s, m, f, D, mode, wantSignal, sc);
 }
 template int stage_kernels_setup<float>(const DevMesh<float> &);
 template int stage_kernels_setup<double>(const DevMesh<double> &);
 template <typename T>
 void launch_update(const DevMesh<T> &m, const Fields<T> &f, const PhysD &D, StageCoef sc, cudaStream_t s) {
-    k_update<T><<<(m.nU + 255) / 256, 256, 0, s>>>(m, f, D, sc);
+    launch_pdl(k_update<T>, (m.nU + 255) / 256, 256, 0, s, m, f, D, sc);
 }
 template <typename T>
 void launch_halo_pack(const T *rec, size_t nRec, int nval, const int32_t *cells, int cnt, T *out,
@@ -868,12 +888,12 @@ void launch_prim(int n, const double *U, T *W, size_t wStride, const PhysD &D, c
     k_prim<T><<<(n + 255) / 256, 256, 0, s>>>(n, U, W, wStride, D);
 }
 void launch_dt_finalize(const double *blockMin, int nBlocks, double cfl, double maxDt, double *dt, cudaStream_t s) {
-    k_dt_finalize<<<1, 1024, 0, s>>>(blockMin, nBlocks, cfl, maxDt, dt);
+    launch_pdl(k_dt_finalize, 1, 1024, 0, s, blockMin, nBlocks, cfl, maxDt, dt);
 }
 void launch_cons(int n, int ivar, const double *U, const double *vol, double *blockSum, double *out, cudaStream_t s) {
     const int nb = cons_blocks(n);
-    k_cons_blocks<<<nb, kConsThreads, 0, s>>>(n, ivar, U, vol, blockSum);
-    k_cons_final<<<1, 1024, 0, s>>>(blockSum, nb, out);
+    launch_pdl(k_cons_blocks, nb, kConsThreads, 0, s, n, ivar, U, vol, blockSum);
+    launch_pdl(k_cons_final, 1, 1024, 0, s, blockSum, nb, out);
 }
 void launch_probe(int n, const double *U, const double *vol, const PhysD &D, double *blockOut, double *out,
                   cudaStream_t s) {

@@ -4,6 +4,31 @@
 
 namespace fg {
 
+// Programmatic dependent launch: the kernels of a step are launched so that a kernel's blocks may become
+// resident while the last blocks of the one before still run.  Rules: every thread of such a kernel
+// calls pdl_wait before it reads anything that an earlier kernel writes, before it writes anything,
+// and before it returns (a grid that finished without waiting would release the next one too early); before
+// pdl_wait a kernel reads the mesh arrays only, which no kernel writes.  pdl_wait returns when the
+// earlier kernels have completed and their writes are visible; pdl_trigger lets the next kernel start.
+// Both do nothing in a kernel launched the ordinary way.  What earlier kernels write is read with ordinary
+// loads: the non-coherent path (__ldg, const __restrict__) is for data that no kernel in flight writes.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... K, typename... A>
+inline void launch_pdl(void (*kernel)(K...), int grid, int block, size_t smem, cudaStream_t s, const A &...args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, K(args)...);   // errors are read by the callers' cudaGetLastError
+}
+
 // Cell-ordered (renumbered) device mesh.  Per-slot arrays are cell-major: a[c * nSlots + k], so
 // the lanes that work on the faces of one cell read contiguous words.
 template <typename T>

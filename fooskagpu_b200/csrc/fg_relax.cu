@@ -406,8 +406,10 @@ __device__ __forceinline__ int needs_chem(const RelaxParams &R, const double *u)
 // relaxation kernel but one runs a single branch
 constexpr int kOrdThreads = 256;
 
-__global__ void k_relax_partition(int n, const double *__restrict__ U, const RelaxParams R, uint8_t *isChem,
+__global__ void k_relax_partition(int n, const double *U, const RelaxParams R, uint8_t *isChem,
                                   int32_t *blockChem) {
+    pdl_trigger();
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     int chem = 0;
     if (c < n) {
@@ -424,6 +426,8 @@ __global__ void k_relax_partition(int n, const double *__restrict__ U, const Rel
 
 // exclusive scan of the per-block counts (one block of 1024 threads), total into *total
 __global__ void k_relax_scan(const int32_t *cnt, int nb, int32_t *off, int32_t *total) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ int32_t sh[1024];
     const int t = threadIdx.x;
     const int per = (nb + 1023) / 1024;
@@ -448,6 +452,8 @@ __global__ void k_relax_scan(const int32_t *cnt, int nb, int32_t *off, int32_t *
 
 __global__ void k_relax_order(int n, const uint8_t *isChem, const int32_t *blockOff, const int32_t *total,
                               int32_t *order) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ int32_t warpChem[kOrdThreads / 32];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -527,6 +533,8 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
                                                const PhysD D, const RelaxParams R, int32_t *counters,
                                                const SurrogateDev S, const int32_t *order, const int32_t *nChem,
                                                const float4 *pred, int32_t *hullOk) {
+    pdl_trigger();
+    pdl_wait();
     const int m = *nChem;
     // base is the same for every thread of the block: the warp collectives below see full warps
     for (int base = blockIdx.x * blockDim.x; base < m; base += gridDim.x * blockDim.x) {
@@ -573,6 +581,8 @@ __global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINB
                                                const int32_t *order, const int32_t *nChem, const float4 *pred,
                                                const int32_t *hullOk) {
     constexpr bool kPolish = kSG && !kPass;   // the polish runs in this kernel
+    pdl_trigger();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool act = i < n;
     const int c = (kOrd && act) ? order[i] : i;
@@ -662,18 +672,18 @@ static void launch_relax_k(int n, double *U, T *W, size_t wStride, const PhysD &
         // the polish inside (launch_relax runs no separate pass with the log on)
         if (S.enabled) {
             if (lg)
-                k_relax<T, true, true, kOrd><<<nb, 128, 0, s>>>(n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
+                launch_pdl(k_relax<T, true, true, kOrd>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
             else if (O->polishPass)
-                k_relax<T, true, false, kOrd, true><<<nb, 128, 0, s>>>(n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
+                launch_pdl(k_relax<T, true, false, kOrd, true>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
             else
-                k_relax<T, true, false, kOrd><<<nb, 128, 0, s>>>(n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
+                launch_pdl(k_relax<T, true, false, kOrd>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
             return;
         }
     }
     if (lg)
-        k_relax<T, false, true, kOrd><<<nb, 128, 0, s>>>(n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
+        launch_pdl(k_relax<T, false, true, kOrd>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
     else
-        k_relax<T, false, false, kOrd><<<nb, 128, 0, s>>>(n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
+        launch_pdl(k_relax<T, false, false, kOrd>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
 }
 
 template <typename T>
@@ -685,9 +695,9 @@ int launch_relax(int n, double *U, T *W, size_t wStride, const PhysD &D, const R
         return 1;
     }
     const int nb = relax_order_blocks(n);
-    k_relax_partition<<<nb, kOrdThreads, 0, s>>>(n, U, R, O.isChem, O.blockCnt);
-    k_relax_scan<<<1, 1024, 0, s>>>(O.blockCnt, nb, O.blockOff, O.total);
-    k_relax_order<<<nb, kOrdThreads, 0, s>>>(n, O.isChem, O.blockOff, O.total, O.order);
+    launch_pdl(k_relax_partition, nb, kOrdThreads, 0, s, n, U, R, O.isChem, O.blockCnt);
+    launch_pdl(k_relax_scan, 1, 1024, 0, s, O.blockCnt, nb, O.blockOff, O.total);
+    launch_pdl(k_relax_order, nb, kOrdThreads, 0, s, n, O.isChem, O.blockOff, O.total, O.order);
     int k = 4;
     if (S.enabled) {
         // the network on the tensor cores for the chemical cells (order[0 .. nChem)), tiles of 128
@@ -696,7 +706,7 @@ int launch_relax(int n, double *U, T *W, size_t wStride, const PhysD &D, const R
                                                                         O.pred, O.hullOk, O.tcErr);
         k++;
         if (O.polishPass && L.count == nullptr) {
-            k_relax_polish<T><<<std::min((n + 127) / 128, 148 * FG_CHEM_SG_MINBLOCKS), 128, 0, s>>>(
+            launch_pdl(k_relax_polish<T>, std::min((n + 127) / 128, 148 * FG_CHEM_SG_MINBLOCKS), 128, 0, s,
                 n, U, W, wStride, D, R, counters, S, O.order, O.total, O.pred, O.hullOk);
             k++;
         }

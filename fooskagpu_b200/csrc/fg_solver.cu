@@ -245,7 +245,11 @@ struct fg_solver {
 
 namespace fg {
 
-__global__ void k_advance_time(const double *dt, double *t) { *t += *dt; }
+__global__ void k_advance_time(const double *dt, double *t) {
+    pdl_trigger();
+    pdl_wait();
+    *t += *dt;
+}
 
 // export variables of DP/export_plt.cu:42-80 per cell (not averaged to the nodes): x y z avfL avfG
 // rho U V W pressure temperature vaporMass |grad rho|, the last from the most recent gradient
@@ -1015,7 +1019,7 @@ struct SolverT : public fg_solver {
     }
     int advance_time(cudaStream_t s) override {
         prof_begin(FG_K_OTHER, s);
-        k_advance_time<<<1, 1, 0, s>>>(dScal.as<double>(), dScal.as<double>() + 1);
+        launch_pdl(k_advance_time, 1, 1, 0, s, dScal.as<double>(), dScal.as<double>() + 1);
         prof_end(s);
         FG_LAUNCH_CHECK("advance_time");
         return FG_OK;
