@@ -173,10 +173,13 @@ __device__ __forceinline__ double chem_gibbs_diff(const RelaxParams &R, const do
 }
 // the step h[q] of unknown q in the Jacobian
 __device__ __forceinline__ double chem_step(double x) { return fabs(x) < 1e-9 ? 1e-10 : 1.e-5 * x; }
-// points from <= q < to: 0 the base point (residuals), 1 .. 3 a, r, e stepped forward (Jacobian columns)
+// points from <= q < to: 0 the base point (residuals), 1 .. 3 a, r, e stepped forward (Jacobian columns).
+// kWide: the points are unrolled, so that the chains of the three stepped points overlap (same arithmetic,
+// more registers).
+template <bool kWide>
 __device__ __forceinline__ void chem_system(const RelaxParams &R, bool m1, double a, double r, double e, double rm, double re,
                                             int from, int to, ChemSystem &S) {
-#pragma unroll 1
+#pragma unroll(kWide ? 4 : 1)
     for (int q = from; q < to; q++) {
         const double aq = q == 1 ? a + chem_step(a) : a;
         const double rq = q == 2 ? r + chem_step(r) : r;
@@ -278,6 +281,7 @@ __device__ int chem_limit_density(const RelaxParams &R, double a, double old, do
 }
 
 // Chemical equilibrium (DP/chemRlx.cu:4-267): damped Newton from the cell's state
+template <bool kWide>
 __device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
     double a, r, e, rm, re;
     bool m1;
@@ -299,7 +303,7 @@ __device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
     for (int itr = 1;; itr++) {
         *iters = itr;
         ChemSystem S;
-        chem_system(R, m1, a, r, e, rm, re, 0, 4, S);
+        chem_system<kWide>(R, m1, a, r, e, rm, re, 0, 4, S);
         double dx[3];
         const double det = chem_direction(S, dx);
         int ab = det == 0;
@@ -365,7 +369,7 @@ __device__ int chem_polish(const RelaxParams &R, double *U, const float *y, doub
     int ok = 0;
     for (int itr = 0; itr <= maxIt; itr++) {
         ChemSystem S;
-        chem_system(R, m1, a, r, e, rm, re, 0, 1, S);
+        chem_system<false>(R, m1, a, r, e, rm, re, 0, 1, S);
         if (!(a > 0 && a < 1 && r > 0 && S.rp > 0)) break;
         if (fabs(S.res[0]) <= relTol * sp && fabs(S.res[1]) <= relTol * sT && fabs(S.res[2]) <= relTol * sg) {
             ok = 1;
@@ -373,7 +377,7 @@ __device__ int chem_polish(const RelaxParams &R, double *U, const float *y, doub
         }
         if (itr == maxIt) break;
         *iters = itr + 1;
-        chem_system(R, m1, a, r, e, rm, re, 1, 4, S);
+        chem_system<false>(R, m1, a, r, e, rm, re, 1, 4, S);
         double dx[3];
         const double det = chem_direction(S, dx);
         if (!(fabs(det) > 0) || !isfinite(det)) break;
@@ -518,6 +522,12 @@ struct InRelax {
 #define FG_CHEM_SG_MINBLOCKS 4
 #endif
 
+// Chemical-first relaxation of few cells: where every cell has its thread resident at 3 blocks per SM the
+// kernel is bound by the longest chain of Gibbs iterations, and takes the unrolled system with
+// 134 registers (bitwise the same states).  16,096 mixed elements: 133 -> 100 us; above the limit, where
+// 3 blocks cost occupancy, the 73,908-tet bubble went 28 -> 34 us with it.
+constexpr int kWideBlocks = 3, kWideCells = 148 * kWideBlocks * 128;
+
 // hullOk[i] of a chemical cell whose polished surrogate solution k_relax_polish accepted
 constexpr int32_t kPolished = 2;
 
@@ -574,8 +584,8 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
     }
 }
 
-template <typename T, bool kSG, bool kLog, bool kOrd, bool kPass = false>
-__global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINBLOCKS : FG_CHEM_MINBLOCKS)
+template <typename T, bool kSG, bool kLog, bool kOrd, bool kPass = false, bool kWide = false>
+__global__ void __launch_bounds__(128, kWide ? kWideBlocks : kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINBLOCKS : FG_CHEM_MINBLOCKS)
                                             : FG_THERM_MINBLOCKS) k_relax(int n, double *U, T *W, size_t wStride, const PhysD D, const RelaxParams R,
                                                int32_t *counters, const SurrogateDev S, const RelaxLog Lg,
                                                const int32_t *order, const int32_t *nChem, const float4 *pred,
@@ -608,7 +618,7 @@ __global__ void __launch_bounds__(128, kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINB
             used = chem_polish(R, u, pr, rm, re, S.relTol, S.polishIters, &pits);
         }
         if (!used) {
-            ab = (kOrd && chem) ? chem_cell(R, u, &its) : therm_cell(R, u, &its);
+            ab = (kOrd && chem) ? chem_cell<kWide>(R, u, &its) : therm_cell(R, u, &its);
         }
         if (kLog && chem && !used && !ab) {
             // training sample: (rho, e, Y) before the solve -> (p, T, alpha, Y_eq) after it
@@ -677,6 +687,13 @@ static void launch_relax_k(int n, double *U, T *W, size_t wStride, const PhysD &
                 launch_pdl(k_relax<T, true, false, kOrd, true>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
             else
                 launch_pdl(k_relax<T, true, false, kOrd>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order, nChem, pred, hull);
+            return;
+        }
+    }
+    if constexpr (kOrd) {
+        if (!lg && n <= kWideCells) {
+            launch_pdl(k_relax<T, false, false, kOrd, false, true>, nb, 128, 0, s, n, U, W, wStride, D, R, counters, S, L, order,
+                       nChem, pred, hull);
             return;
         }
     }

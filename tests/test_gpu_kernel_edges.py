@@ -64,6 +64,28 @@ def test_gibbs_newton_with_stiffened_gas(pinf_gas):
     assert err.max() < 1e-11, err   # as the relaxation parity: round-off of the same iterates
 
 
+def test_relaxation_kernels_agree_bitwise():
+    """57,798 cells take the relaxation kernel of many cells, the two parts of the mesh (28,899 each) that of
+    few: the same states bit for bit."""
+    nm = meshgen.box_hexes(39, 39, 38, L=(39e-3, 39e-3, 38e-3))
+    m = Mesh.build(nm.nodes, nm.elems, nm.bcs)
+    c = cases.reference_case()
+    U = cases.perturbed_two_phase_ic(c, m.arrays()["cellCenter"], seed=4, vel=25.0)
+    s = Solver(m, c, precision="mixed")
+    s.set_state(U)
+    assert s.relaxation()["nChem"] > 1000
+    whole = s.get_state()
+    s.close()
+    for p in range(2):
+        part = m.partition(2, p)
+        own = part.partition_maps()["cell_global"][:part.n_owned]
+        s = Solver(part, c, precision="mixed")
+        s.set_state(U[own])
+        s.relaxation()
+        assert np.array_equal(s.get_state(), whole[own])
+        s.close()
+
+
 # a tile holds 32 samples, a pass over the blocks 296 tiles
 @pytest.mark.parametrize("n", [1, 31, 33, 296 * 32 + 1])
 def test_training_gradient_batch_sizes(n):
