@@ -205,9 +205,9 @@ int flux_blocks(int n);   // blocks of the gather kernel (= entries of blockMin)
 // relaxation (FP64 Newton), writes U and the primitive record
 struct RelaxParams {
     double gam[2], pinf[2], cp[2], eta[2], satConst[2];
-    // derived per phase: gam - 1, gam pinf, (gam - 1) eta, Cv = Cp / gam, Cv (gam - 1); and of the
+    // derived per phase: gam - 1, gam pinf, (gam - 1) eta, Cv = Cp / gam, Cv (gam - 1) and its reciprocal; of the
     // saturation line f(T) = ((satA + etaT2(P)) satQ + ...) + satB / T + satC log10 T
-    double gm1[2], gpinf[2], gm1eta[2], cv[2], cvgm1[2];
+    double gm1[2], gpinf[2], gm1eta[2], cv[2], cvgm1[2], icvgm1[2];
     double satA, satQ, satB, satC, satD;
     double avfMin, chemLimit, thermUrf, chemUrf, satTempUrf;
     int thermItrMax, chemItrMax, chemFlag;

@@ -17,10 +17,19 @@ namespace fg {
 
 namespace {
 
+// The Newtons are compiled into several kernels (with and without the surrogate, for few and for many
+// cells), whose states agree bitwise: where a product has more than one use, or two products meet in a
+// sum, the roundings are written out, so that no instantiation contracts them its own way.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+// a b - c d
+__device__ __forceinline__ double diff_rn(double a, double b, double c, double d) { return fma_rn(a, b, -mul_rn(c, d)); }
+
 // pressure and temperature of phase m at density r and internal energy e (DP/eqos.h); the phase
 // constants are precomputed once per launch (RelaxParams)
 __device__ __forceinline__ double p_of(const RelaxParams &R, int m, double r, double e) {
-    return R.gm1[m] * r * e - R.gpinf[m] - R.gm1eta[m] * r;
+    return fma_rn(-R.gm1eta[m], r, fma_rn(mul_rn(R.gm1[m], r), e, -R.gpinf[m]));
 }
 __device__ __forceinline__ double t_of(const RelaxParams &R, int m, double r, double e) {
     return (p_of(R, m, r, e) + R.pinf[m]) / (R.cvgm1[m] * r);
@@ -31,9 +40,9 @@ __device__ __forceinline__ double t_of(const RelaxParams &R, int m, double r, do
 // 1e-3 .. 1e-8 of itself, and the series gives that change directly, without the cancellation of
 // two logarithms and at a tenth of the cost of the second one
 constexpr double kLog10e = 0.43429448190325182765, kSmallLog = 1e-3;
-__device__ __forceinline__ double log10_1p(double d) {
-    const double s = 1.0 + d * (-1.0 / 2 + d * (1.0 / 3 + d * (-1.0 / 4 + d * (1.0 / 5 + d * (-1.0 / 6)))));
-    return (kLog10e * d) * s;
+__device__ __forceinline__ double log10_1p(double d, double base = 0.0) {
+    const double s = fma_rn(d, fma_rn(d, fma_rn(d, fma_rn(d, fma_rn(d, -1.0 / 6, 1.0 / 5), -1.0 / 4), 1.0 / 3), -1.0 / 2), 1.0);
+    return fma_rn(mul_rn(kLog10e, d), s, base);   // base + log10(1 + d)
 }
 
 // Newton on the saturation temperature (DP/relaxation.cu:4-38) with the reference's forward
@@ -63,9 +72,13 @@ __device__ double sat_temp(const RelaxParams &R, double P, double temp, double u
 // Thermal (p, T) equilibrium (DP/thermRlx.cu:4-235).  The unknowns are the density r and energy e of
 // the minor phase; the primary phase follows from volume and energy.  The two solved phases are
 // named minor / primary and mapped to the phases 0 / 1 by selects, so no array is indexed at run
-// time; the energy difference reuses the densities and their reciprocals, and each iteration takes
-// 11 divisions where the reference's order of operations takes 23 (981 k-tet bubble, 8.6 iterations
-// per cell: 255 -> 162 us; 2.0 M-cell jet: 241 -> 158 us).
+// time.  Divisions are what an iteration costs, and it takes 4 of them (the reference's order of
+// operations 23): with s = part_minor / r the primary density is part / (1 - s), so its reciprocal needs
+// none; the stepped density is r (1 + 1e-4), so 1 / r and s scale by a constant; and the Newton step is
+// solved for in units of the difference steps, so the Jacobian's columns stay differences.
+// Bound by FP64 instructions.  981 k-tet bubble (8.6 iterations per cell): 255 us in the reference's order,
+// 159 with shared denominators (11 divisions), 113 now; 2.0 M-cell jet 241, 145, 116; 128^3 TGV (one
+// iteration) 141, 112, 111.
 __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
     const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
     const double a1 = 1 - a0;
@@ -89,38 +102,38 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
     int aborted = 0;
     for (int itr = 1;; itr++) {
         *iters = itr;
-        // residuals at (r, e)
-        double rp = arp / (1 - arm / r);
+        // residuals at (r, e); i0, i1: reciprocals of Cv (g - 1) rho
+        const double ir = 1.0 / r, sh = mul_rn(arm, ir);
+        double rp = arp * (1.0 / (1 - sh)), irp = (1 - sh) * iarp;
         const double ep = enp - iarp * (arm * (e - enm));
-        const double i0 = 1.0 / (R.cvgm1[0] * (m1 ? rp : r)), i1 = 1.0 / (R.cvgm1[1] * (m1 ? r : rp));
+        const double i0 = R.icvgm1[0] * (m1 ? irp : ir), i1 = R.icvgm1[1] * (m1 ? ir : irp);
         double p0 = p_of(R, 0, m1 ? rp : r, m1 ? ep : e), p1 = p_of(R, 1, m1 ? r : rp, m1 ? e : ep);
-        const double res0 = p0 - p1, res1 = (p0 + R.pinf[0]) * i0 - (p1 + R.pinf[1]) * i1;
+        const double res0 = p0 - p1, res1 = diff_rn(p0 + R.pinf[0], i0, p1 + R.pinf[1], i1);
         const bool inside = r > 0.0 && rp > 0.0;
         // forward differences in e (same densities), then in r (same energies)
-        const double he = 1e-4 * e, hr = 1e-4 * r;
-        double j01, j11, j00, j10;
+        const double he = mul_rn(1e-4, e), hr = mul_rn(1e-4, r);
+        double d01, d11, d00, d10;
         {
-            const double eq = e + he, epq = enp - iarp * (arm * (eq - enm));
+            const double eq = add_rn(e, he), epq = enp - iarp * (arm * (eq - enm));
             p0 = p_of(R, 0, m1 ? rp : r, m1 ? epq : eq);
             p1 = p_of(R, 1, m1 ? r : rp, m1 ? eq : epq);
-            const double ih = 1.0 / he;
-            j01 = ((p0 - p1) - res0) * ih;
-            j11 = (((p0 + R.pinf[0]) * i0 - (p1 + R.pinf[1]) * i1) - res1) * ih;
+            d01 = (p0 - p1) - res0;
+            d11 = diff_rn(p0 + R.pinf[0], i0, p1 + R.pinf[1], i1) - res1;
         }
         {
-            const double rq = r + hr;
-            rp = arp / (1 - arm / rq);
-            const double x0 = m1 ? rp : rq, x1 = m1 ? rq : rp;
-            p0 = p_of(R, 0, x0, m1 ? ep : e);
-            p1 = p_of(R, 1, x1, m1 ? e : ep);
-            const double ih = 1.0 / hr;
-            j00 = ((p0 - p1) - res0) * ih;
-            j10 = (((p0 + R.pinf[0]) / (R.cvgm1[0] * x0) - (p1 + R.pinf[1]) / (R.cvgm1[1] * x1)) - res1) * ih;
+            constexpr double kStep = 1.0 / (1.0 + 1e-4);
+            const double rq = add_rn(r, hr), irq = ir * kStep, sq = mul_rn(sh, kStep);
+            rp = arp * (1.0 / (1 - sq));
+            irp = (1 - sq) * iarp;
+            p0 = p_of(R, 0, m1 ? rp : rq, m1 ? ep : e);
+            p1 = p_of(R, 1, m1 ? rq : rp, m1 ? e : ep);
+            d00 = (p0 - p1) - res0;
+            d10 = diff_rn(p0 + R.pinf[0], R.icvgm1[0] * (m1 ? irp : irq), p1 + R.pinf[1], R.icvgm1[1] * (m1 ? irq : irp)) - res1;
         }
-        const double det = j00 * j11 - j10 * j01;
-        const bool bad = isnan(j00) || isnan(j01) || isnan(j10) || isnan(j11) || det == 0;
+        const double det = diff_rn(d00, d11, d10, d01);
+        const bool bad = isnan(d00) || isnan(d01) || isnan(d10) || isnan(d11) || det == 0;
         if (!bad && inside) {
-            const float chk = sqrt(res0 * res0 + res1 * res1);
+            const float chk = sqrt(fma_rn(res0, res0, mul_rn(res1, res1)));
             if (chk < minRes) {
                 minRes = chk;
                 br = r;
@@ -134,8 +147,8 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
             break;
         }
         const double id = R.thermUrf / det;
-        r = r - id * (j11 * res0 - j01 * res1);
-        e = e - id * (j00 * res1 - j10 * res0);
+        r = fma_rn(-hr, mul_rn(id, diff_rn(d11, res0, d01, res1)), r);
+        e = fma_rn(-he, mul_rn(id, diff_rn(d00, res1, d10, res0)), e);
         if (!(fabs(res0) > 1.e-2) && !(fabs(res1) > 1.e-2)) break;
     }
     const double rp = arp / (1 - arm / r);
@@ -152,27 +165,31 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
 // The reference's entropy log10(T^g / (p + pinf)^(g - 1)) is evaluated as g log10 T - (g - 1)
 // log10(p + pinf), with no powers; the logarithms are taken once, at the base point, and the three
 // perturbed points add log10 of the ratio from the series (log10_1p), or logarithms of their own
-// where the ratio is not near 1: 4 logarithms an iteration in place of 12 and 16 powers.  Bound by FP64
-// instructions (and, on few cells, by the latency of one cell's chain of iterations): the relaxation
-// kernel went 784 -> 241 us on a 61 x 67 x 59 box with 36 % chemical cells, 331 -> 130 us on 16,096 cells
-// of mixed elements, and 387 -> 119 us on a 64^3 box with the surrogate's polish.
+// where the ratio is not near 1: 4 logarithms an iteration in place of 12 and 16 powers.  A point reuses
+// the reciprocals that its step leaves alone, and the Newton step is solved for in units of the difference
+// steps: 10 divisions in place of 26.  Bound by FP64 instructions and, on few cells, by the latency of one
+// cell's chain of iterations: the relaxation kernel takes 241 us (784 in the reference's order) on a
+// 61 x 67 x 59 box with 36 % chemical cells, 79 (331) on 16,096 mixed elements, and 106 (387) on a 64^3 box
+// with the surrogate's polish.
 struct ChemLog {
     double lT[2], lP[2], lG;   // log10 of T, p + pinf of the phases, and of the gas pressure
 };
 struct ChemSystem {
-    double res[3], jac[3][3];
+    double res[3], dif[3][3];   // residuals; dif[i][q]: change of residual i by step q
     double ap, rp;   // volume fraction and density of the primary phase at the base point
-    // the base point: pressures, temperatures, reciprocals of T and p + pinf, logarithms
+    // the base point: reciprocals of the primary phase's volume fraction and partial density and of r,
+    // pressures, temperatures, reciprocals of T and p + pinf, logarithms
+    double iap, ipart, ir;
     double p[2], T[2], iT[2], iP[2];
     ChemLog log;
 };
 __device__ __forceinline__ double chem_gibbs_diff(const RelaxParams &R, const double *T, const ChemLog &l) {
-    const double s0 = R.cv[0] * (R.gam[0] * l.lT[0] - R.gm1[0] * l.lP[0]);
-    const double s1 = R.cv[1] * (R.gam[1] * l.lT[1] - R.gm1[1] * l.lP[1]) + (R.satConst[0] * l.lG + R.satConst[1]);
-    return (R.cp[0] * T[0] + R.eta[0] - T[0] * s0) - (R.cp[1] * T[1] + R.eta[1] - T[1] * s1);
+    const double s0 = mul_rn(R.cv[0], diff_rn(R.gam[0], l.lT[0], R.gm1[0], l.lP[0]));
+    const double s1 = fma_rn(R.cv[1], diff_rn(R.gam[1], l.lT[1], R.gm1[1], l.lP[1]), fma_rn(R.satConst[0], l.lG, R.satConst[1]));
+    return fma_rn(-T[0], s0, fma_rn(R.cp[0], T[0], R.eta[0])) - fma_rn(-T[1], s1, fma_rn(R.cp[1], T[1], R.eta[1]));
 }
 // the step h[q] of unknown q in the Jacobian
-__device__ __forceinline__ double chem_step(double x) { return fabs(x) < 1e-9 ? 1e-10 : 1.e-5 * x; }
+__device__ __forceinline__ double chem_step(double x) { return fabs(x) < 1e-9 ? 1e-10 : mul_rn(1.e-5, x); }
 // points from <= q < to: 0 the base point (residuals), 1 .. 3 a, r, e stepped forward (Jacobian columns).
 // kWide: the points are unrolled, so that the chains of the three stepped points overlap (same arithmetic,
 // more registers).
@@ -181,25 +198,29 @@ __device__ __forceinline__ void chem_system(const RelaxParams &R, bool m1, doubl
                                             int from, int to, ChemSystem &S) {
 #pragma unroll(kWide ? 4 : 1)
     for (int q = from; q < to; q++) {
-        const double aq = q == 1 ? a + chem_step(a) : a;
-        const double rq = q == 2 ? r + chem_step(r) : r;
-        const double eq = q == 3 ? e + chem_step(e) : e;
-        const double ap = 1 - aq, part = rm - aq * rq;
-        const double rp = part / ap, ep = (re - aq * rq * eq) / part;
+        const double aq = q == 1 ? add_rn(a, chem_step(a)) : a;
+        const double rq = q == 2 ? add_rn(r, chem_step(r)) : r;
+        const double eq = q == 3 ? add_rn(e, chem_step(e)) : e;
+        // a step in a, r or e leaves the reciprocals that do not contain it as they are
+        const double ap = 1 - aq, mq = mul_rn(aq, rq), part = add_rn(rm, -mq);
+        const double iap = q < 2 ? 1.0 / ap : S.iap;
+        const double ipart = q < 3 ? 1.0 / part : S.ipart;
+        const double ir = (q & 1) || q > 2 ? S.ir : 1.0 / rq;
+        const double rp = part * iap, irp = ap * ipart, ep = mul_rn(fma_rn(-mq, eq, re), ipart);
         const double x0 = m1 ? rp : rq, x1 = m1 ? rq : rp;
         double p[2], T[2];
         p[0] = p_of(R, 0, x0, m1 ? ep : eq);
         p[1] = p_of(R, 1, x1, m1 ? eq : ep);
-        T[0] = (p[0] + R.pinf[0]) / (R.cvgm1[0] * x0);
-        T[1] = (p[1] + R.pinf[1]) / (R.cvgm1[1] * x1);
+        T[0] = (p[0] + R.pinf[0]) * (R.icvgm1[0] * (m1 ? irp : ir));
+        T[1] = (p[1] + R.pinf[1]) * (R.icvgm1[1] * (m1 ? ir : irp));
         ChemLog l;
         const double d0 = (T[0] - S.T[0]) * S.iT[0], d1 = (T[1] - S.T[1]) * S.iT[1];
         const double d2 = (p[0] - S.p[0]) * S.iP[0], d3 = (p[1] - S.p[1]) * S.iP[1];
         if (q && fabs(d0) < kSmallLog && fabs(d1) < kSmallLog && fabs(d2) < kSmallLog && fabs(d3) < kSmallLog) {
-            l.lT[0] = S.log.lT[0] + log10_1p(d0);
-            l.lT[1] = S.log.lT[1] + log10_1p(d1);
-            l.lP[0] = S.log.lP[0] + log10_1p(d2);
-            l.lP[1] = S.log.lP[1] + log10_1p(d3);
+            l.lT[0] = log10_1p(d0, S.log.lT[0]);
+            l.lT[1] = log10_1p(d1, S.log.lT[1]);
+            l.lP[0] = log10_1p(d2, S.log.lP[0]);
+            l.lP[1] = log10_1p(d3, S.log.lP[1]);
         } else {
             l.lT[0] = log10(T[0]);
             l.lT[1] = log10(T[1]);
@@ -219,41 +240,44 @@ __device__ __forceinline__ void chem_system(const RelaxParams &R, bool m1, doubl
             for (int m = 0; m < 2; m++) {
                 S.p[m] = p[m];
                 S.T[m] = T[m];
-                S.iT[m] = 1.0 / T[m];
                 S.iP[m] = 1.0 / (p[m] + R.pinf[m]);
+                S.iT[m] = S.iP[m] * (R.cvgm1[m] * (m ? x1 : x0));
             }
+            S.iap = iap;
+            S.ipart = ipart;
+            S.ir = ir;
         } else {
-            const double ih = 1.0 / chem_step(q == 1 ? a : (q == 2 ? r : e));
-            const double c0 = ((p[0] - p[1]) - S.res[0]) * ih, c1 = ((T[0] - T[1]) - S.res[1]) * ih, c2 = (g - S.res[2]) * ih;
-            if (q == 1) { S.jac[0][0] = c0; S.jac[1][0] = c1; S.jac[2][0] = c2; }
-            if (q == 2) { S.jac[0][1] = c0; S.jac[1][1] = c1; S.jac[2][1] = c2; }
-            if (q == 3) { S.jac[0][2] = c0; S.jac[1][2] = c1; S.jac[2][2] = c2; }
+            const double c0 = (p[0] - p[1]) - S.res[0], c1 = (T[0] - T[1]) - S.res[1], c2 = g - S.res[2];
+            if (q == 1) { S.dif[0][0] = c0; S.dif[1][0] = c1; S.dif[2][0] = c2; }
+            if (q == 2) { S.dif[0][1] = c0; S.dif[1][1] = c1; S.dif[2][1] = c2; }
+            if (q == 3) { S.dif[0][2] = c0; S.dif[1][2] = c1; S.dif[2][2] = c2; }
         }
     }
 }
 
-// dx = jac^-1 res by cofactors; the determinant
-__device__ __forceinline__ double chem_direction(const ChemSystem &S, double *dx) {
-    const double(*j)[3] = S.jac;
-    const double c00 = j[1][1] * j[2][2] - j[1][2] * j[2][1];
-    const double c01 = j[1][0] * j[2][2] - j[1][2] * j[2][0];
-    const double c02 = j[1][0] * j[2][1] - j[1][1] * j[2][0];
-    const double det = j[0][0] * c00 - j[0][1] * c01 + j[0][2] * c02;
+// dx = J^-1 res at (a, r, e), by cofactors and in units of the difference steps; the determinant of
+// the differences
+__device__ __forceinline__ double chem_direction(const ChemSystem &S, double a, double r, double e, double *dx) {
+    const double(*j)[3] = S.dif;
+    const double c00 = diff_rn(j[1][1], j[2][2], j[1][2], j[2][1]);
+    const double c01 = diff_rn(j[1][2], j[2][0], j[1][0], j[2][2]);
+    const double c02 = diff_rn(j[1][0], j[2][1], j[1][1], j[2][0]);
+    const double det = fma_rn(j[0][0], c00, fma_rn(j[0][1], c01, mul_rn(j[0][2], c02)));
     const double id = 1.0 / det;
-    dx[0] = id * (c00 * S.res[0] - (j[0][1] * j[2][2] - j[0][2] * j[2][1]) * S.res[1] +
-                  (j[0][1] * j[1][2] - j[0][2] * j[1][1]) * S.res[2]);
-    dx[1] = id * (-c01 * S.res[0] + (j[0][0] * j[2][2] - j[0][2] * j[2][0]) * S.res[1] -
-                  (j[0][0] * j[1][2] - j[0][2] * j[1][0]) * S.res[2]);
-    dx[2] = id * (c02 * S.res[0] - (j[0][0] * j[2][1] - j[0][1] * j[2][0]) * S.res[1] +
-                  (j[0][0] * j[1][1] - j[0][1] * j[1][0]) * S.res[2]);
+    auto row = [&](double h, double x, double y, double z) {
+        return mul_rn(mul_rn(h, id), fma_rn(x, S.res[0], fma_rn(y, S.res[1], mul_rn(z, S.res[2]))));
+    };
+    dx[0] = row(chem_step(a), c00, diff_rn(j[0][2], j[2][1], j[0][1], j[2][2]), diff_rn(j[0][1], j[1][2], j[0][2], j[1][1]));
+    dx[1] = row(chem_step(r), c01, diff_rn(j[0][0], j[2][2], j[0][2], j[2][0]), diff_rn(j[0][2], j[1][0], j[0][0], j[1][2]));
+    dx[2] = row(chem_step(e), c02, diff_rn(j[0][1], j[2][0], j[0][0], j[2][1]), diff_rn(j[0][0], j[1][1], j[0][1], j[1][0]));
     return det;
 }
 
 // relaxed state from the minor phase's (a, r, e): the primary phase closes mass and energy
 __device__ __forceinline__ void chem_store(const RelaxParams &R, bool m1, double a, double r, double e, double rm, double re,
                                            double *U) {
-    const double part = rm - a * r;
-    const double ap = 1 - a, rp = part / ap, ep = (re - a * r * e) / part;
+    const double mq = mul_rn(a, r), part = add_rn(rm, -mq);
+    const double ap = 1 - a, rp = part / ap, ep = fma_rn(-mq, e, re) / part;
     const double x0 = m1 ? ap : a, r0 = m1 ? rp : r, r1 = m1 ? r : rp, e0 = m1 ? ep : e, e1 = m1 ? e : ep;
     const double x1 = m1 ? a : ap;
     U[0] = fmin(fmax(R.avfMin / 100, x0), 1 - R.avfMin / 100);
@@ -305,14 +329,14 @@ __device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
         ChemSystem S;
         chem_system<kWide>(R, m1, a, r, e, rm, re, 0, 4, S);
         double dx[3];
-        const double det = chem_direction(S, dx);
+        const double det = chem_direction(S, a, r, e, dx);
         int ab = det == 0;
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) ab |= isnan(S.jac[i][j]);
+            for (int j = 0; j < 3; j++) ab |= isnan(S.dif[i][j]);
         if (!ab && a > 0.0 && a < 1.0 && S.ap > 0.0 && S.ap < 1.0 && r > 0.0 && S.rp > 0.0) {
-            const float chk = sqrt(S.res[0] * S.res[0] + S.res[1] * S.res[1] + S.res[2] * S.res[2]);
+            const float chk = sqrt(fma_rn(S.res[0], S.res[0], fma_rn(S.res[1], S.res[1], mul_rn(S.res[2], S.res[2]))));
             if (chk < minRes) {
                 minRes = chk;
                 ba = a;
@@ -321,11 +345,11 @@ __device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
             }
         }
         const double oa = a, orr = r;
-        a = a - R.chemUrf * dx[0];
+        a = fma_rn(-R.chemUrf, dx[0], a);
         ab |= chem_limit_fraction(R, oa, a, dx[0]);
-        r = r - R.chemUrf * dx[1];
+        r = fma_rn(-R.chemUrf, dx[1], r);
         ab |= chem_limit_density(R, a, orr, r, dx[1], rm);
-        e = e - R.chemUrf * dx[2];
+        e = fma_rn(-R.chemUrf, dx[2], e);
         if (ab || itr > R.chemItrMax) {
             a = ba;
             r = br;
@@ -379,7 +403,7 @@ __device__ int chem_polish(const RelaxParams &R, double *U, const float *y, doub
         *iters = itr + 1;
         chem_system<false>(R, m1, a, r, e, rm, re, 1, 4, S);
         double dx[3];
-        const double det = chem_direction(S, dx);
+        const double det = chem_direction(S, a, r, e, dx);
         if (!(fabs(det) > 0) || !isfinite(det)) break;
         a -= dx[0];
         r -= dx[1];
@@ -502,18 +526,15 @@ struct InRelax {
     }
 };
 
-// resident blocks asked of the compiler for the thermal-only instantiation (kOrd false): its
-// FP64 Newton is latency-bound; 6 blocks of 128 threads (80 registers, a few spilled) measured
-// 0.180 -> 0.150 ms early and 0.461 -> 0.400 ms later in the 128^3 TGV against 4 blocks
+// resident blocks asked of the compiler for the thermal-only instantiation (kOrd false): 6 blocks of 128
+// threads (80 registers) 114.5 us per relaxation of the 128^3 TGV, 7 blocks 115.7, 8 blocks 117.3
 #ifndef FG_THERM_MINBLOCKS
 #define FG_THERM_MINBLOCKS 6
 #endif
-// the same for the chemical-first instantiations (kOrd true: Gibbs and thermal Newton).  Without
-// the surrogate 6 blocks (85 registers) measured 0.770 -> 0.730 ms per relaxation on a 64^3
-// two-phase box (39 % chemical cells) and 1.321 -> 1.157 ms on the 4 M-tet bubble (almost all
-// thermal) against 4 blocks (5 and 7 were slower on the box); uncapped (156-196 registers) was
-// 2.81 ms against 1.99 at 4 blocks on the 96^3 box.  With the surrogate's polish path 4 blocks
-// (128 registers) measured 0.81 -> 0.66 ms against uncapped on that box.  The same budget serves
+// the same for the chemical-first instantiations (kOrd true: Gibbs and thermal Newton).  Without the
+// surrogate, on the box with 36 % chemical cells / the 981 k-tet bubble (almost all thermal): 4 blocks 257 /
+// 188 us, 5 blocks 228 / 170, 6 blocks 235 / 160, 8 blocks 254 / 156.  With the surrogate's polish, on the
+// 64^3 box: 4 blocks (128 registers) 119 us, 5 blocks 130, 6 blocks 133; the same budget serves
 // k_relax_polish, the surrogate's polish as a pass of its own.
 #ifndef FG_CHEM_MINBLOCKS
 #define FG_CHEM_MINBLOCKS 6
@@ -524,7 +545,7 @@ struct InRelax {
 
 // Chemical-first relaxation of few cells: where every cell has its thread resident at 3 blocks per SM the
 // kernel is bound by the longest chain of Gibbs iterations, and takes the unrolled system with
-// 134 registers (bitwise the same states).  16,096 mixed elements: 133 -> 100 us; above the limit, where
+// 157 registers (bitwise the same states).  16,096 mixed elements: 133 -> 100 us; above the limit, where
 // 3 blocks cost occupancy, the 73,908-tet bubble went 28 -> 34 us with it.
 constexpr int kWideBlocks = 3, kWideCells = 148 * kWideBlocks * 128;
 

@@ -369,6 +369,7 @@ struct SolverT : public fg_solver {
             R.gm1eta[k] = (g - 1) * cs.eta[k];
             R.cv[k] = cs.Cp[k] / g;
             R.cvgm1[k] = (cs.Cp[k] / g) * (g - 1);
+            R.icvgm1[k] = 1.0 / R.cvgm1[k];
         }
         {
             // saturation line (DP/relaxation.cu:4-38)
