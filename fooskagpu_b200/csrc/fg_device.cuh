@@ -95,7 +95,7 @@ __device__ __forceinline__ void w_store(T *base, size_t stride, int c, const T *
 
 // The gradient records G use the same component-major layout with vectors of 16 or 32 bytes per
 // precision: 32-byte vectors halve the vector loads of the face kernel (256-bit
-// ld.global.nc.v4.f64 / v8.f32).  FP64 records (36 values = 9 vectors of 4) take them: the FP64
+// ld.global.v4.f64 / v8.f32).  FP64 records (36 values = 9 vectors of 4) take them: the FP64
 // face kernel measured 1-2 % faster; FP32 records would need padding to 40 values, and the FP32
 // face kernel measured 5 % slower with them.  grec_alloc<T>() values per cell are allocated.
 #ifndef FG_G_VEC_BYTES_F

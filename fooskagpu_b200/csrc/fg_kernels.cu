@@ -119,7 +119,7 @@ __device__ __forceinline__ T limiter_phi(T num, T diff) {
 // 86 -> 78 (981 k tets); FP64 224 -> 213 (96^3 hexes), 123 -> 109 (480 k tets).
 template <typename T, int kLim, int S>
 __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_grad(const DevMesh<T> m, const T *W,
-                                                                T *G, const PhysT<T> P) {
+                                                                T *G, const PhysT<T> P, double *time, const double *dt) {
     using V = typename Vec16<T>::type;
     constexpr int B = StageCells<T>::value, WQ = stage_w_vecs<T>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -153,6 +153,8 @@ __global__ void __launch_bounds__(StageCells<T>::value, MinBlocks<T>::grad) k_gr
         }
     }
     pdl_wait();
+    // first stage of a step: physical time advances by the previous dt (DP/explicitLoop.cu:29)
+    if (time && b == 0 && t == 0) *time += *dt;
     for (int r = threadIdx.x; r < nRec; r += B) {
         if (r < B && r >= nBlockRecs) continue;
         const int src = r < B ? lo + r : (r < 2 * B ? id1 : m.haloIds[hs + r - B]);
@@ -545,15 +547,17 @@ __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gat
 
 // CFL bound of the own cells from their maximum face signal speed (k_face with wantSignal 2), as
 // the gather kernel computes it on the residual path: signal[c], then the deterministic block
-// minimum of volP / signal over blocks of the gather kernel's size
+// minimum of volP / signal over blocks of the gather kernel's size.  reset: the maxima are left at zero for
+// the next dt step.
 template <typename T>
-__global__ void k_cell_cfl(const DevMesh<T> m, const T *cellSig, double *signal, double *blockMin) {
+__global__ void k_cell_cfl(const DevMesh<T> m, T *cellSig, double *signal, double *blockMin, int reset) {
     pdl_trigger();
     pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double cfl = 1e12;
     if (c < m.nU) {
         const T sig = cellSig[c];
+        if (reset) cellSig[c] = 0;
         signal[c] = (double)sig;
         cfl = m.volP[c] / (double)sig;
     }
@@ -843,7 +847,7 @@ void launch_grad(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, cud
     const size_t sm = grad_smem<T>(m.blockCells + m.maxHalo);
     auto *k = m.nSlots == 4 ? (P.limiter == 1 ? k_grad<T, 1, 4> : k_grad<T, 0, 4>)
                             : (P.limiter == 1 ? k_grad<T, 1, 6> : k_grad<T, 0, 6>);
-    launch_pdl(k, nb, m.blockCells, sm, s, m, f.Win, f.G, P);
+    launch_pdl(k, nb, m.blockCells, sm, s, m, f.Win, f.G, P, f.time, f.dt);
 }
 template <typename T>
 void launch_face(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, int wantSignal, cudaStream_t s) {
@@ -852,8 +856,8 @@ void launch_face(const DevMesh<T> &m, const Fields<T> &f, const PhysT<T> &P, int
                f.cellSig, P, wantSignal);
 }
 template <typename T>
-void launch_cell_cfl(const DevMesh<T> &m, const Fields<T> &f, cudaStream_t s) {
-    launch_pdl(k_cell_cfl<T>, flux_blocks(m.nU), kGatherThreads, 0, s, m, f.cellSig, f.signal, f.blockMin);
+void launch_cell_cfl(const DevMesh<T> &m, const Fields<T> &f, int reset, cudaStream_t s) {
+    launch_pdl(k_cell_cfl<T>, flux_blocks(m.nU), kGatherThreads, 0, s, m, f.cellSig, f.signal, f.blockMin, reset);
 }
 template <typename T>
 void launch_gather(const DevMesh<T> &m, const Fields<T> &f, const PhysD &D, int mode, int wantSignal,
@@ -922,8 +926,8 @@ template void launch_grad<float>(const DevMesh<float> &, const Fields<float> &, 
 template void launch_grad<double>(const DevMesh<double> &, const Fields<double> &, const PhysT<double> &, cudaStream_t);
 template void launch_face<float>(const DevMesh<float> &, const Fields<float> &, const PhysT<float> &, int, cudaStream_t);
 template void launch_face<double>(const DevMesh<double> &, const Fields<double> &, const PhysT<double> &, int, cudaStream_t);
-template void launch_cell_cfl<float>(const DevMesh<float> &, const Fields<float> &, cudaStream_t);
-template void launch_cell_cfl<double>(const DevMesh<double> &, const Fields<double> &, cudaStream_t);
+template void launch_cell_cfl<float>(const DevMesh<float> &, const Fields<float> &, int, cudaStream_t);
+template void launch_cell_cfl<double>(const DevMesh<double> &, const Fields<double> &, int, cudaStream_t);
 template void launch_gather<float>(const DevMesh<float> &, const Fields<float> &, const PhysD &, int, int, StageCoef, cudaStream_t);
 template void launch_gather<double>(const DevMesh<double> &, const Fields<double> &, const PhysD &, int, int, StageCoef, cudaStream_t);
 template void launch_update<float>(const DevMesh<float> &, const Fields<float> &, const PhysD &, StageCoef, cudaStream_t);

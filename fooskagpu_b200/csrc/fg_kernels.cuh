@@ -38,7 +38,6 @@ struct DevMesh {
     int nG;             // cells with gradients: own cells, then a part's first-layer ghosts
     int nFEval;         // faces the face kernel evaluates (those touching an own cell) come first
     int nSlots;         // slots per cell: 4 (tets only) or 6
-    const int32_t *nbr;   // neighbour cell, or -bc (1..5) on a boundary slot, or INT32_MIN unused
     const int32_t *flags; // bits 0-2: faces of the cell; bit 3+k: cell owns the face of slot k
     // the six per-slot geometry arrays below are consecutive blocks of geoStride values, in this
     // order, starting at aox; geoStride >= n * nSlots is a multiple of 16 bytes so that every
@@ -119,8 +118,7 @@ template <typename T> struct MinBlocks {
 #ifndef FG_GRAD_MINB_D
 #define FG_GRAD_MINB_D 6
 #endif
-// FP64 face kernel: 6 resident blocks of 64 (168 registers, 88 bytes of spill) measured 15 % faster
-// than the compiler's 200 registers (5 blocks) on the 128^3 hex workload
+// FP64 face kernel (96^3 hexes): 6 resident blocks of 64 (168 registers) 329 us, 5 blocks 338, 8 blocks 366
 #ifndef FG_FACE_MINB_D
 #define FG_FACE_MINB_D 6
 #endif
@@ -144,9 +142,10 @@ struct Fields {
     T *G;               // limiter + gradient records (GREC values per cell, component-major vectors of
                         // gvec_bytes<T>() bytes, grec_alloc<T>() values per cell allocated)
     double *signal;     // [n]
-    T *cellSig;         // [n] per-cell maximum face signal speed of a dt step (zeroed before it)
+    T *cellSig;         // [n] per-cell maximum face signal speed of a dt step (zero before it)
     double *blockMin;   // [nBlocks]
     double *dt;         // device scalar
+    double *time;       // device scalar that the gradient kernel advances by dt, null for none
     int32_t *bad;       // set to the step counter + 1 when an updated state is not finite or its
                         // mixture density is not positive (sticky until cleared; mapped host memory)
     int32_t step;       // the step counter the kernels record
@@ -197,7 +196,7 @@ void launch_halo_unpack(T *rec, size_t nRec, int nval, const int32_t *cells, int
 // dt steps of the fused path: per cell (own cells, blocks of the gather kernel) the CFL bound
 // volP / cellSig and the signal, the block minima into blockMin[flux_blocks(nU)]
 template <typename T>
-void launch_cell_cfl(const DevMesh<T> &m, const Fields<T> &f, cudaStream_t s);
+void launch_cell_cfl(const DevMesh<T> &m, const Fields<T> &f, int reset, cudaStream_t s);
 // dt = min(cfl * min_blocks, maxDt) from blockMin[nBlocks]
 void launch_dt_finalize(const double *blockMin, int nBlocks, double cfl, double maxDt, double *dt, cudaStream_t s);
 int flux_blocks(int n);   // blocks of the gather kernel (= entries of blockMin)

@@ -190,6 +190,7 @@ struct fg_solver {
     fg_halo_ops halo{};       // the partitioned run's transport (fg_solver_set_halo)
     void *haloSend = nullptr, *haloRecv = nullptr;
     int iStep = 0;
+    bool advanceTime = false;   // the next gradient pass advances the physical time (start of a step)
     uint64_t bytes = 0;
     virtual int init(const fg::Mesh &m) = 0;
     // gradient pass only; face fluxes + gather (+ RK unless mode is the residual) only
@@ -232,7 +233,6 @@ struct fg_solver {
     virtual int relax_counts(fg_relax_stats *st) = 0;
     virtual int cons(int ivar, double *out, cudaStream_t s) = 0;
     virtual int probe(double *out4, cudaStream_t s) = 0;
-    virtual int advance_time(cudaStream_t s) = 0;
     virtual int get_time(double *dt, double *t) = 0;
     virtual int set_dt(double dt) = 0;
     virtual int set_time(double t) = 0;
@@ -244,12 +244,6 @@ struct fg_solver {
 };
 
 namespace fg {
-
-__global__ void k_advance_time(const double *dt, double *t) {
-    pdl_trigger();
-    pdl_wait();
-    *t += *dt;
-}
 
 // export variables of DP/export_plt.cu:42-80 per cell (not averaged to the nodes): x y z avfL avfG
 // rho U V W pressure temperature vaporMass |grad rho|, the last from the most recent gradient
@@ -292,10 +286,12 @@ __global__ void k_field_vars(int n, const double *__restrict__ U, const T *__res
 // automatic surrogate polish pass: a separate pass when fewer than one cell in kSparseChemInv of
 // the previous surrogate relaxation was chemical
 constexpr int kSparseChemInv = 10;
+// most cells of a mesh whose per-cell signal maxima are reset by the CFL kernel (see dt_stage)
+constexpr int kResetCells = 1 << 18;
 
 template <typename T>
 struct SolverT : public fg_solver {
-    DevBuf dNbr, dFlags, dGeo, dVol, dVolP, dIVol, dNew2Old, dHaloStart, dHaloIds, dSlotLocal;
+    DevBuf dFlags, dGeo, dVol, dVolP, dIVol, dNew2Old, dHaloStart, dHaloIds, dSlotLocal;
     DevBuf dU, dU0, dRHS, dW[2], dG, dSig, dCellSig, dBlockMin, dScal, dCnt, dCons, dStage;
     DevBuf dStageIn;   // staging buffer of the asynchronous uploads (on first use)
     DevBuf dStageOut[2];   // staging buffers of the asynchronous downloads (on first use)
@@ -325,6 +321,7 @@ struct SolverT : public fg_solver {
         f.cellSig = dCellSig.as<T>();
         f.blockMin = dBlockMin.as<double>();
         f.dt = dScal.as<double>();
+        f.time = advanceTime ? dScal.as<double>() + 1 : nullptr;
         f.bad = dBad;
         f.step = iStep;
         return f;
@@ -590,7 +587,6 @@ struct SolverT : public fg_solver {
         dm.haloStart = dHaloStart.as<int32_t>();
         dm.haloIds = dHaloIds.as<int32_t>();
         dm.slotLocal = dSlotLocal.as<int16_t>();
-        FG_CUDA_TRY(dNbr.alloc(S * sizeof(int32_t)));
         FG_CUDA_TRY(dFlags.alloc((size_t)n * sizeof(int32_t)));
         FG_CUDA_TRY(dGeo.alloc(6 * GS * sizeof(T)));
         FG_CUDA_TRY(dVol.alloc((size_t)n * sizeof(double)));
@@ -598,7 +594,6 @@ struct SolverT : public fg_solver {
         FG_CUDA_TRY(dIVol.alloc((size_t)n * sizeof(double)));
         FG_CUDA_TRY(cudaMemcpy(dIVol.p, ivol.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(dNew2Old.alloc((size_t)n * sizeof(int32_t)));
-        FG_CUDA_TRY(cudaMemcpy(dNbr.p, nbr.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dFlags.p, flags.data(), (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dGeo.p, geo.data(), 6 * GS * sizeof(T), cudaMemcpyHostToDevice));
         FG_CUDA_TRY(cudaMemcpy(dVol.p, vol.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
@@ -626,6 +621,7 @@ struct SolverT : public fg_solver {
         FG_CUDA_TRY(dG.alloc((size_t)n * grec_alloc<T>() * sizeof(T)));
         FG_CUDA_TRY(dSig.alloc((size_t)n * sizeof(double)));
         FG_CUDA_TRY(dCellSig.alloc((size_t)n * sizeof(T)));
+        FG_CUDA_TRY(cudaMemset(dCellSig.p, 0, (size_t)n * sizeof(T)));
         FG_CUDA_TRY(dBlockMin.alloc((size_t)std::max(flux_blocks(n), cons_blocks(n)) * sizeof(double)));
         FG_CUDA_TRY(dScal.alloc(4 * sizeof(double)));   // dt, time, cons
         FG_CUDA_TRY(dCnt.alloc(8 * sizeof(int32_t)));
@@ -648,7 +644,7 @@ struct SolverT : public fg_solver {
         const double scal[4] = {cs.dt, 0.0, 0.0, 0.0};
         FG_CUDA_TRY(cudaMemcpy(dScal.p, scal, sizeof(scal), cudaMemcpyHostToDevice));
         bytes = 0;
-        for (DevBuf *b : {&dNbr, &dFlags, &dGeo, &dVol, &dVolP, &dIVol, &dNew2Old, &dU, &dU0, &dRHS, &dStage, &dW[0], &dW[1], &dG,
+        for (DevBuf *b : {&dFlags, &dGeo, &dVol, &dVolP, &dIVol, &dNew2Old, &dU, &dU0, &dRHS, &dStage, &dW[0], &dW[1], &dG,
                           &dSig, &dCellSig, &dBlockMin, &dScal, &dCnt, &dHaloStart, &dHaloIds, &dSlotLocal, &dFIdx, &dFGeo,
                           &dSlotFace, &dClosure, &dFB, &dOrdFlag, &dOrdCnt, &dOrdOff, &dOrder, &dOrdTotal,
                           &dPred, &dHullOk, &dTcErr})
@@ -658,7 +654,6 @@ struct SolverT : public fg_solver {
         dm.nG = nG;
         dm.nFEval = nFEval;
         dm.nSlots = nSlots;
-        dm.nbr = dNbr.as<int32_t>();
         dm.flags = dFlags.as<int32_t>();
         T *g = dGeo.as<T>();
         dm.geoStride = GS;
@@ -794,6 +789,7 @@ struct SolverT : public fg_solver {
         prof_begin(FG_K_GRAD, s);
         launch_grad<T>(dm, f, P, s);
         prof_end(s);
+        advanceTime = false;
         FG_LAUNCH_CHECK("gradients");
         return FG_OK;
     }
@@ -886,12 +882,18 @@ struct SolverT : public fg_solver {
         int rc;
         if ((rc = gradients_halo(s))) return rc;
         Fields<T> f = fields(cur);
-        FG_CUDA_TRY(cudaMemsetAsync(dCellSig.p, 0, (size_t)n * sizeof(T), s));
+        // Zero maxima before the face kernel: left so by the last dt step's CFL kernel on small meshes, where
+        // a memset between the gradient and the face kernel would end their overlap (8^3 TGV run 290 ->
+        // 272 us, 73,908-tet bubble 979 -> 947, both with the time advance in the gradient kernel); by a memset
+        // on large ones, which also brings the array into L2 for the face kernel's atomics (without it 480 k
+        // tets 9.24 -> 9.36 ms, 2.0 M cells 10.52 -> 10.72 ms; 262 k cells 1806 -> 1794 us).
+        const bool reset = n <= kResetCells;
+        if (!reset) FG_CUDA_TRY(cudaMemsetAsync(dCellSig.p, 0, (size_t)n * sizeof(T), s));
         prof_begin(FG_K_FLUX, s);
         launch_face<T>(dm, f, P, 2, s);
         prof_end(s);
         prof_begin(FG_K_DT, s);
-        launch_cell_cfl<T>(dm, f, s);
+        launch_cell_cfl<T>(dm, f, reset, s);
         prof_end(s);
         FG_LAUNCH_CHECK("cell cfl");
         if ((rc = time_step(nullptr, s))) return rc;
@@ -1016,13 +1018,6 @@ struct SolverT : public fg_solver {
             FG_CUDA_TRY(cudaMemcpyAsync(out, o, sizeof(double), cudaMemcpyDeviceToHost, s));
             FG_CUDA_TRY(cudaStreamSynchronize(s));
         }
-        return FG_OK;
-    }
-    int advance_time(cudaStream_t s) override {
-        prof_begin(FG_K_OTHER, s);
-        launch_pdl(k_advance_time, 1, 1, 0, s, dScal.as<double>(), dScal.as<double>() + 1);
-        prof_end(s);
-        FG_LAUNCH_CHECK("advance_time");
         return FG_OK;
     }
     int get_time(double *dt, double *t) override {
@@ -1564,16 +1559,20 @@ int fg_step(fg_solver *s, void *stream) {
     if (s->hBad[0] || s->hBad[1]) return s->flag_error();
     cudaStream_t st = (cudaStream_t)stream;
     const fg_case &c = s->cs;
-    int rc = s->advance_time(st);   // physicalTime += dt (previous dt, DP/explicitLoop.cu:29)
-    if (rc) return rc;
+    int rc;
+    s->advanceTime = true;   // physicalTime += dt (previous dt, DP/explicitLoop.cu:29)
     const int rk = c.rkSteps;
     for (int irk = 0; irk < rk; irk++) {
         const int writeU0 = (rk == 3 && irk == 0);
         if (c.adaptDt == 1 && irk == 0 && s->iStep % c.adaptDtItr == 0) {
             // residual with the signal speeds, new dt, then the stage update (DP/explicitLoop.cu:45-47)
-            if ((rc = s->dt_stage(irk, writeU0, st))) return rc;
+            rc = s->dt_stage(irk, writeU0, st);
         } else {
-            if ((rc = s->stage(irk, writeU0, st))) return rc;
+            rc = s->stage(irk, writeU0, st);
+        }
+        if (rc) {
+            s->advanceTime = false;
+            return rc;
         }
     }
     if (c.relaxFlag == 0)
