@@ -199,23 +199,40 @@ __device__ __forceinline__ T eos_c2(const PhysT<T> &P, int m, T rho, T p) {
     return (P.gam[m] * (p + P.pinf[m])) / rho;
 }
 
-// FP64 cons -> prim at the cell centre (DP/cons2prim.h:2-24), rounded to T for storage.  Written with
-// the partial quantities (rho_L e_L = U[6] / alpha, rho = U[1] + U[2]): three divisions instead of the
-// nine of the reference's order, and fewer roundings in the pressures.
+// FP64 cons -> prim at the cell centre (DP/cons2prim.h:2-24), rounded to S for storage.  FP64 records take the
+// reference's order of operations.  FP32 records, which round at 6e-8, are written with the partial quantities
+// (rho_L e_L = U[6] / alpha, rho = U[1] + U[2]): three divisions instead of nine.  In FP64 they move the
+// pressures by a rounding, and with it the states that the thermal Newton stops at (see therm_cell_ordered), for
+// 2 us of the gather kernel's 122 (96^3 TGV).
 template <typename S>
 __device__ __forceinline__ void cons2prim_d(const PhysD &D, const double *U, S *w) {
     const double a = fmin(fmax(D.avfLo, U[0]), D.avfHi);
-    const double ia = 1.0 / a, ig = 1.0 / (1 - a), ir = 1.0 / (U[1] + U[2]);
-    const double rl = U[1] * ia, rg = U[2] * ig;
     w[0] = (S)a;
-    w[1] = (S)rl;
-    w[2] = (S)rg;
-    w[3] = (S)(U[3] * ir);
-    w[4] = (S)(U[4] * ir);
-    w[5] = (S)(U[5] * ir);
-    w[6] = (S)(D.gm1[0] * (U[6] * ia) - D.gpinf[0] - D.gm1eta[0] * rl);
-    w[7] = (S)(D.gm1[1] * (U[7] * ig) - D.gpinf[1] - D.gm1eta[1] * rg);
     w[8] = (S)U[9];
+    if constexpr (sizeof(S) == 8) {
+        const double rl = U[1] / a;
+        const double rg = U[2] / (1 - a);
+        const double rho = a * rl + (1 - a) * rg;
+        const double el = U[6] / (a * rl);
+        const double eg = U[7] / ((1 - a) * rg);
+        w[1] = (S)rl;
+        w[2] = (S)rg;
+        w[3] = (S)(U[3] / rho);
+        w[4] = (S)(U[4] / rho);
+        w[5] = (S)(U[5] / rho);
+        w[6] = (S)(D.gm1[0] * rl * el - D.gpinf[0] - D.gm1eta[0] * rl);
+        w[7] = (S)(D.gm1[1] * rg * eg - D.gpinf[1] - D.gm1eta[1] * rg);
+    } else {
+        const double ia = 1.0 / a, ig = 1.0 / (1 - a), ir = 1.0 / (U[1] + U[2]);
+        const double rl = U[1] * ia, rg = U[2] * ig;
+        w[1] = (S)rl;
+        w[2] = (S)rg;
+        w[3] = (S)(U[3] * ir);
+        w[4] = (S)(U[4] * ir);
+        w[5] = (S)(U[5] * ir);
+        w[6] = (S)(D.gm1[0] * (U[6] * ia) - D.gpinf[0] - D.gm1eta[0] * rl);
+        w[7] = (S)(D.gm1[1] * (U[7] * ig) - D.gpinf[1] - D.gm1eta[1] * rg);
+    }
 }
 
 // Boundary ghost of a primitive state (DP/bc.h:78-84).  bc: 1 symmetry, 2 outlet, 3 inlet,
@@ -291,7 +308,12 @@ __device__ __forceinline__ void hllc_flux(const PhysT<T> &P, const T *L, const T
     const T un = left ? uL : uR;
     const T cK = left ? SL : SR;
     const T pm = left ? pmL : pmR;
-    const T rho = left ? rL : rR;
+    T rho = left ? rL : rR;
+    if constexpr (sizeof(T) == 8) {
+        // the roundings of FP64 results, written out (see cons2prim_d): the right state's density takes the
+        // liquid's product unrounded
+        if (!left) rho = __fma_rn(R[0], R[1], __dmul_rn(1 - R[0], R[2]));
+    }
     // prim2cons (DP/prim2cons.h:2-21)
     const T c1 = s[0] * s[1];
     const T c2 = (1 - s[0]) * s[2];

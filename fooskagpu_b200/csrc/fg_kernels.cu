@@ -449,8 +449,8 @@ __device__ __forceinline__ void load_slot_faces(const int32_t *__restrict__ p, i
 }
 
 // S: slots per cell (4 or 6).  The face ids of all slots come first, in 8- or 16-byte loads, so that the
-// record of a face does not wait for its id in turn (with the fewer divisions of cons2prim_d, FP64 96^3
-// TGV: 165 -> 133 us; FP32 is bound by memory at 128^3, 201 us, and by this chain on few cells).
+// record of a face does not wait for its id in turn (FP64 96^3 TGV, with the face records in planes: 164 -> 122 us;
+// FP32 is bound by memory at 128^3, 201 us, and by this chain on few cells).
 template <typename T, int S>
 __global__ void __launch_bounds__(FG_GATHER_THREADS, MinBlocks<T>::gather) k_gather(const DevMesh<T> m, Fields<T> f, const PhysD D, int mode,
                                                 int wantSignal, StageCoef sc) {

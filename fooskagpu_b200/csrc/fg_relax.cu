@@ -159,6 +159,92 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
     return aborted;
 }
 
+// The same Newton in the reference's order of operations, for FP64 runs.  The Newton stops at the absolute residual
+// 1e-2 after one more step under-relaxed by thermUrf, so two orders of operations that put a residual on either
+// side of it leave states about (1 - thermUrf) 1e-2 apart in pressure: 2.5e-5 of the vortex's p of about 70, where
+// FP64 results are otherwise alike to 1e-15.  With the rearranged Newton (and cons2prim_d) 16 FP64 vortex boxes of
+// 1,386 to 340,860 cells were 4e-9 to 1.3e-6 off in the norm after 2 to 4 steps.  FP64 runs are what other
+// results are checked against, and keep the one order; the roundings are written out, so that every kernel that
+// this is compiled into agrees.  20 divisions per iteration: relaxation of the 96^3 TGV 55 us, 51 rearranged.
+__device__ int therm_cell_ordered(const RelaxParams &R, double *U, int *iters) {
+    const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
+    const double a1 = 1 - a0;
+    const double rho0 = U[1] / a0, rho1 = U[2] / a1;
+    const double ar0 = mul_rn(a0, rho0), ar1 = mul_rn(a1, rho1);
+    const double e0 = U[6] / ar0, e1 = U[7] / ar1;
+    const bool m1 = !(a1 > a0);   // the minor phase is phase 1
+    const double arm = m1 ? ar1 : ar0, arp = m1 ? ar0 : ar1;
+    double r = m1 ? rho1 : rho0, e = m1 ? e1 : e0;
+    double enm, enp;
+    {
+        const double rm = add_rn(ar0, ar1);
+        const double u = U[3] / rm, v = U[4] / rm, w = U[5] / rm;
+        const double de = fma_rn(-0.5, fma_rn(w, w, fma_rn(u, u, mul_rn(v, v))),
+                                 fma_rn(-(ar1 / rm), e1, fma_rn(-(ar0 / rm), e0, U[8] / rm)));
+        enm = add_rn(e, de);
+        enp = add_rn(m1 ? e0 : e1, de);
+    }
+    const double iarp = 1 / arp;
+    // the primary phase's density and energy, and the residuals, at the minor phase's (r, e)
+    auto close = [&](double rq, double eq, double &rp, double &ep) {
+        rp = mul_rn(1 / (1 - arm / rq), arp);
+        ep = fma_rn(-iarp, mul_rn(arm, eq - enm), enp);
+    };
+    auto point = [&](double rq, double eq, double &rp, double &d0, double &d1) {
+        double ep;
+        close(rq, eq, rp, ep);
+        const double x0 = m1 ? rp : rq, x1 = m1 ? rq : rp;
+        const double p0 = p_of(R, 0, x0, m1 ? ep : eq), p1 = p_of(R, 1, x1, m1 ? eq : ep);
+        d0 = p0 - p1;
+        d1 = (p0 + R.pinf[0]) / mul_rn(R.cvgm1[0], x0) - (p1 + R.pinf[1]) / mul_rn(R.cvgm1[1], x1);
+    };
+    double br = r, be = e;   // best iterate
+    float minRes = 1e9f;
+    int aborted = 0;
+    for (int itr = 1;; itr++) {
+        *iters = itr;
+        double rp, res0, res1, j00, j10, j01, j11;
+        point(r, e, rp, res0, res1);
+        const double hr = mul_rn(1e-4, r);
+        r = add_rn(r, hr);
+        point(r, e, rp, j00, j10);
+        r = add_rn(r, -hr);   // not always the value it was
+        j00 = (j00 - res0) / hr;
+        j10 = (j10 - res1) / hr;
+        const double he = mul_rn(1e-4, e);
+        e = add_rn(e, he);
+        point(r, e, rp, j01, j11);
+        e = add_rn(e, -he);
+        j01 = (j01 - res0) / he;
+        j11 = (j11 - res1) / he;
+        const double det = diff_rn(j00, j11, j10, j01);
+        const bool bad = isnan(j00) || isnan(j01) || isnan(j10) || isnan(j11) || det == 0;
+        if (!bad && r > 0.0 && rp > 0.0) {
+            const float chk = sqrt(fma_rn(res0, res0, mul_rn(res1, res1)));
+            if (chk < minRes) {
+                minRes = chk;
+                br = r;
+                be = e;
+            }
+        }
+        if (bad || itr > R.thermItrMax) {
+            r = br;
+            e = be;
+            aborted = 1;
+            break;
+        }
+        r = fma_rn(-R.thermUrf, fma_rn(j11 / det, res0, mul_rn(-j01 / det, res1)), r);
+        e = fma_rn(-R.thermUrf, fma_rn(-j10 / det, res0, mul_rn(j00 / det, res1)), e);
+        if (!(fabs(res0) > 1.e-2) && !(fabs(res1) > 1.e-2)) break;
+    }
+    double rp, ep;
+    close(r, e, rp, ep);
+    U[0] = fmin(fmax(R.avfMin / 100, ar0 / (m1 ? rp : r)), 1 - R.avfMin / 100);
+    U[6] = ar0 * (m1 ? ep : e);
+    U[7] = ar1 * (m1 ? e : ep);
+    return aborted;
+}
+
 // Residuals of the chemical (p, T, Gibbs) equilibrium of a cell with mixture density rm and internal
 // energy re per unit volume (DP/chemRlx.cu:4-130), and their forward-difference Jacobian.  The
 // unknowns are volume fraction a, density r and energy e of the minor phase (phase 1 if m1).
@@ -639,7 +725,8 @@ __global__ void __launch_bounds__(128, kWide ? kWideBlocks : kOrd ? ((kSG && !kP
             used = chem_polish(R, u, pr, rm, re, S.relTol, S.polishIters, &pits);
         }
         if (!used) {
-            ab = (kOrd && chem) ? chem_cell<kWide>(R, u, &its) : therm_cell(R, u, &its);
+            if (kOrd && chem) ab = chem_cell<kWide>(R, u, &its);
+            else ab = sizeof(T) == 8 ? therm_cell_ordered(R, u, &its) : therm_cell(R, u, &its);
         }
         if (kLog && chem && !used && !ab) {
             // training sample: (rho, e, Y) before the solve -> (p, T, alpha, Y_eq) after it

@@ -1,6 +1,9 @@
 """Sizes and branches at which the stage, relaxation and training kernels change path, against the
 oracle: last blocks of 4-slot (tets) and 6-slot meshes, a gas phase with its own p_inf in the Gibbs
 Newton, training batches that do not fill a tile or a pass over the blocks."""
+import math
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -62,6 +65,29 @@ def test_gibbs_newton_with_stiffened_gas(pinf_gas):
     s.close()
     assert st["nChem"] > 50 and {k: sg[k] for k in st} == st
     assert err.max() < 1e-11, err   # as the relaxation parity: round-off of the same iterates
+
+
+@pytest.mark.parametrize("box", [(5, 6, 7), (8, 8, 8)])
+def test_fp64_vortex_keeps_its_stop_decisions(box):
+    """Four FP64 vortex steps against stored states.  The thermal Newton stops at an absolute residual, so a change
+    of rounding anywhere in a step lets some cells stop one iterate earlier or later, which moves the pressure by
+    about (1 - thermUrf) 1e-2 / 70 = 3e-5 (a rearranged Newton: 1.1e-4 and 2.6e-5 here); states whose every
+    cell stops where it did agree to rounding, 1e-12 with room."""
+    L = 2 * math.pi
+    nm = meshgen.box_hexes(*box, L=(L, L, L), side_bc={})
+    m = Mesh.build(nm.nodes, nm.elems, nm.bcs, periodic=(L, L, L))
+    c = cases.tgv_case()
+    c.adaptDtItr = 2
+    c.hllcTieTol = 1e-9
+    s = Solver(m, c, precision="fp64")
+    s.set_state(cases.tgv_ic(c, m.arrays()["cellCenter"] + np.array([0.3, 1.1, 2.0])))
+    for _ in range(4):
+        s.step()
+    U = s.get_state()
+    s.close()
+    ref = np.load(Path(__file__).parent / "golden" / "tgv_fp64_steps.npz")["%d_%d_%d" % box]
+    err = np.abs(U - ref).max(axis=0) / np.maximum(np.abs(ref).max(axis=0), 1e-300)
+    assert err.max() < 1e-12, err
 
 
 def test_relaxation_kernels_agree_bitwise():
