@@ -199,6 +199,12 @@ __device__ __forceinline__ T eos_c2(const PhysT<T> &P, int m, T rho, T p) {
     return (P.gam[m] * (p + P.pinf[m])) / rho;
 }
 
+// operations that the compiler neither contracts nor takes apart
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 // FP64 cons -> prim at the cell centre (DP/cons2prim.h:2-24), rounded to S for storage.  FP64 records take the
 // reference's order of operations.  FP32 records, which round at 6e-8, are written with the partial quantities
 // (rho_L e_L = U[6] / alpha, rho = U[1] + U[2]): three divisions instead of nine.  In FP64 they move the
@@ -212,26 +218,25 @@ __device__ __forceinline__ void cons2prim_d(const PhysD &D, const double *U, S *
     if constexpr (sizeof(S) == 8) {
         const double rl = U[1] / a;
         const double rg = U[2] / (1 - a);
-        const double rho = a * rl + (1 - a) * rg;
-        const double el = U[6] / (a * rl);
-        const double eg = U[7] / ((1 - a) * rg);
+        const double al = mul_rn(a, rl), ag = mul_rn(1 - a, rg), rho = add_rn(al, ag);
+        const double el = U[6] / al, eg = U[7] / ag;
         w[1] = (S)rl;
         w[2] = (S)rg;
         w[3] = (S)(U[3] / rho);
         w[4] = (S)(U[4] / rho);
         w[5] = (S)(U[5] / rho);
-        w[6] = (S)(D.gm1[0] * rl * el - D.gpinf[0] - D.gm1eta[0] * rl);
-        w[7] = (S)(D.gm1[1] * rg * eg - D.gpinf[1] - D.gm1eta[1] * rg);
+        w[6] = (S)fma_rn(-D.gm1eta[0], rl, fma_rn(mul_rn(D.gm1[0], rl), el, -D.gpinf[0]));
+        w[7] = (S)fma_rn(-D.gm1eta[1], rg, fma_rn(mul_rn(D.gm1[1], rg), eg, -D.gpinf[1]));
     } else {
         const double ia = 1.0 / a, ig = 1.0 / (1 - a), ir = 1.0 / (U[1] + U[2]);
-        const double rl = U[1] * ia, rg = U[2] * ig;
+        const double rl = mul_rn(U[1], ia), rg = mul_rn(U[2], ig);
         w[1] = (S)rl;
         w[2] = (S)rg;
         w[3] = (S)(U[3] * ir);
         w[4] = (S)(U[4] * ir);
         w[5] = (S)(U[5] * ir);
-        w[6] = (S)(D.gm1[0] * (U[6] * ia) - D.gpinf[0] - D.gm1eta[0] * rl);
-        w[7] = (S)(D.gm1[1] * (U[7] * ig) - D.gpinf[1] - D.gm1eta[1] * rg);
+        w[6] = (S)fma_rn(-D.gm1eta[0], rl, fma_rn(D.gm1[0], mul_rn(U[6], ia), -D.gpinf[0]));
+        w[7] = (S)fma_rn(-D.gm1eta[1], rg, fma_rn(D.gm1[1], mul_rn(U[7], ig), -D.gpinf[1]));
     }
 }
 
@@ -312,7 +317,7 @@ __device__ __forceinline__ void hllc_flux(const PhysT<T> &P, const T *L, const T
     if constexpr (sizeof(T) == 8) {
         // the roundings of FP64 results, written out (see cons2prim_d): the right state's density takes the
         // liquid's product unrounded
-        if (!left) rho = __fma_rn(R[0], R[1], __dmul_rn(1 - R[0], R[2]));
+        if (!left) rho = fma_rn(R[0], R[1], mul_rn(1 - R[0], R[2]));
     }
     // prim2cons (DP/prim2cons.h:2-21)
     const T c1 = s[0] * s[1];

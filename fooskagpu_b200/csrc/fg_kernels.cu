@@ -271,9 +271,6 @@ __device__ __forceinline__ void face_state(const T *w, const T *g, T dx, T dy, T
     }
 }
 
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-
 // gradient of the liquid-phase temperature T = (p_L + pInf) / (cv (gamma - 1) rho_L) of a cell from
 // its record and gradients (chain rule), added to acc.  The product is rounded before the sum, so that the
 // sum over a face's two cells does not depend on which comes first (a part of a partitioned mesh may

@@ -20,9 +20,9 @@ namespace {
 // The Newtons are compiled into several kernels (with and without the surrogate, for few and for many
 // cells), whose states agree bitwise: where a product has more than one use, or two products meet in a
 // sum, the roundings are written out, so that no instantiation contracts them its own way.
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// u^2 + v^2 + w^2
+__device__ __forceinline__ double sq_rn(double u, double v, double w) { return fma_rn(w, w, fma_rn(u, u, mul_rn(v, v))); }
 // a b - c d
 __device__ __forceinline__ double diff_rn(double a, double b, double c, double d) { return fma_rn(a, b, -mul_rn(c, d)); }
 
@@ -83,18 +83,19 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
     const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
     const double a1 = 1 - a0;
     const double rho0 = U[1] / a0, rho1 = U[2] / a1;
-    const double ar0 = a0 * rho0, ar1 = a1 * rho1;
+    const double ar0 = mul_rn(a0, rho0), ar1 = mul_rn(a1, rho1);
     const double e0 = U[6] / ar0, e1 = U[7] / ar1;
     const bool m1 = !(a1 > a0);   // the minor phase is phase 1
     const double arm = m1 ? ar1 : ar0, arp = m1 ? ar0 : ar1;
     double r = m1 ? rho1 : rho0, e = m1 ? e1 : e0;
     double enm, enp;
     {
-        const double im = 1.0 / (ar0 + ar1);
-        const double u = U[3] * im, v = U[4] * im, w = U[5] * im;
-        const double de = U[8] * im - (ar0 * im) * e0 - (ar1 * im) * e1 - 0.5 * (u * u + v * v + w * w);
-        enm = e + de;
-        enp = (m1 ? e0 : e1) + de;
+        const double im = 1.0 / add_rn(ar0, ar1);
+        const double u = mul_rn(U[3], im), v = mul_rn(U[4], im), w = mul_rn(U[5], im);
+        const double de = fma_rn(-0.5, sq_rn(u, v, w),
+                                 fma_rn(-mul_rn(ar1, im), e1, fma_rn(U[8], im, -mul_rn(mul_rn(ar0, im), e0))));
+        enm = add_rn(e, de);
+        enp = add_rn(m1 ? e0 : e1, de);
     }
     const double iarp = 1.0 / arp;
     double br = r, be = e;   // best iterate
@@ -105,7 +106,7 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
         // residuals at (r, e); i0, i1: reciprocals of Cv (g - 1) rho
         const double ir = 1.0 / r, sh = mul_rn(arm, ir);
         double rp = arp * (1.0 / (1 - sh)), irp = (1 - sh) * iarp;
-        const double ep = enp - iarp * (arm * (e - enm));
+        const double ep = fma_rn(-iarp, mul_rn(arm, e - enm), enp);
         const double i0 = R.icvgm1[0] * (m1 ? irp : ir), i1 = R.icvgm1[1] * (m1 ? ir : irp);
         double p0 = p_of(R, 0, m1 ? rp : r, m1 ? ep : e), p1 = p_of(R, 1, m1 ? r : rp, m1 ? e : ep);
         const double res0 = p0 - p1, res1 = diff_rn(p0 + R.pinf[0], i0, p1 + R.pinf[1], i1);
@@ -114,7 +115,7 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
         const double he = mul_rn(1e-4, e), hr = mul_rn(1e-4, r);
         double d01, d11, d00, d10;
         {
-            const double eq = add_rn(e, he), epq = enp - iarp * (arm * (eq - enm));
+            const double eq = add_rn(e, he), epq = fma_rn(-iarp, mul_rn(arm, eq - enm), enp);
             p0 = p_of(R, 0, m1 ? rp : r, m1 ? epq : eq);
             p1 = p_of(R, 1, m1 ? r : rp, m1 ? eq : epq);
             d01 = (p0 - p1) - res0;
@@ -152,7 +153,7 @@ __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
         if (!(fabs(res0) > 1.e-2) && !(fabs(res1) > 1.e-2)) break;
     }
     const double rp = arp / (1 - arm / r);
-    const double ep = enp - iarp * (arm * (e - enm));
+    const double ep = fma_rn(-iarp, mul_rn(arm, e - enm), enp);
     U[0] = fmin(fmax(R.avfMin / 100, ar0 / (m1 ? rp : r)), 1 - R.avfMin / 100);
     U[6] = ar0 * (m1 ? ep : e);
     U[7] = ar1 * (m1 ? e : ep);
@@ -179,7 +180,7 @@ __device__ int therm_cell_ordered(const RelaxParams &R, double *U, int *iters) {
     {
         const double rm = add_rn(ar0, ar1);
         const double u = U[3] / rm, v = U[4] / rm, w = U[5] / rm;
-        const double de = fma_rn(-0.5, fma_rn(w, w, fma_rn(u, u, mul_rn(v, v))),
+        const double de = fma_rn(-0.5, sq_rn(u, v, w),
                                  fma_rn(-(ar1 / rm), e1, fma_rn(-(ar0 / rm), e0, U[8] / rm)));
         enm = add_rn(e, de);
         enp = add_rn(m1 ? e0 : e1, de);
@@ -378,16 +379,35 @@ __device__ __forceinline__ void chem_store(const RelaxParams &R, bool m1, double
 // fractions in [0, 1], partial densities in [0, rm].  1 where it stays outside.
 __device__ int chem_limit_fraction(const RelaxParams &R, double old, double &x, double dx) {
     float urf = (float)R.chemUrf;
-    if (x < 0) { while (x < R.chemLimit && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; } }
-    if (x > 1) { while (x > 1.0 - R.chemLimit && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; } }
+    if (x < 0) { while (x < R.chemLimit && urf > 0.0005f) { urf = urf / 2; x = fma_rn(-(double)urf, dx, old); } }
+    if (x > 1) { while (x > 1.0 - R.chemLimit && urf > 0.0005f) { urf = urf / 2; x = fma_rn(-(double)urf, dx, old); } }
     return x < 0 || x > 1;
 }
 __device__ int chem_limit_density(const RelaxParams &R, double a, double old, double &x, double dx, double rm) {
     float urf = (float)R.chemUrf;
     double ar = a * x;
-    if (x < 0) { while (x < 0 && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; } }
-    if (ar > rm) { while (ar > rm && urf > 0.0005f) { urf = urf / 2; x = old - urf * dx; ar = a * x; } }
+    if (x < 0) { while (x < 0 && urf > 0.0005f) { urf = urf / 2; x = fma_rn(-(double)urf, dx, old); } }
+    if (ar > rm) { while (ar > rm && urf > 0.0005f) { urf = urf / 2; x = fma_rn(-(double)urf, dx, old); ar = a * x; } }
     return x < 0 || ar > rm;
+}
+
+// mixture density and internal energy per unit volume of a cell, and the phases it starts from: volume fractions,
+// densities and partial densities
+struct ChemMix {
+    double a0, a1, r0, r1, ar0, ar1, rm, re;
+};
+__device__ __forceinline__ ChemMix chem_mixture(const RelaxParams &R, const double *U) {
+    ChemMix m;
+    m.a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
+    m.a1 = 1 - m.a0;
+    m.r0 = U[1] / m.a0;
+    m.r1 = U[2] / m.a1;
+    m.ar0 = mul_rn(m.a0, m.r0);
+    m.ar1 = mul_rn(m.a1, m.r1);
+    m.rm = add_rn(m.ar0, m.ar1);
+    const double u = U[3] / m.rm, v = U[4] / m.rm, w = U[5] / m.rm;
+    m.re = fma_rn(-mul_rn(0.5, m.rm), sq_rn(u, v, w), U[8]);
+    return m;
 }
 
 // Chemical equilibrium (DP/chemRlx.cu:4-267): damped Newton from the cell's state
@@ -396,16 +416,13 @@ __device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
     double a, r, e, rm, re;
     bool m1;
     {
-        const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100), a1 = 1 - a0;
-        const double r0 = U[1] / a0, r1 = U[2] / a1;
-        const double e0 = U[6] / (a0 * r0), e1 = U[7] / (a1 * r1);
-        rm = a0 * r0 + a1 * r1;
-        const double u = U[3] / rm, v = U[4] / rm, w = U[5] / rm;
-        re = U[8] - 0.5 * rm * (u * u + v * v + w * w);
-        m1 = !(a1 > a0);
-        a = m1 ? a1 : a0;
-        r = m1 ? r1 : r0;
-        e = m1 ? e1 : e0;
+        const ChemMix m = chem_mixture(R, U);
+        rm = m.rm;
+        re = m.re;
+        m1 = !(m.a1 > m.a0);
+        a = m1 ? m.a1 : m.a0;
+        r = m1 ? m.r1 : m.r0;
+        e = m1 ? U[7] / m.ar1 : U[6] / m.ar0;
     }
     double ba = a, br = r, be = e;   // best iterate
     float minRes = 1e9f;
@@ -447,18 +464,6 @@ __device__ int chem_cell(const RelaxParams &R, double *U, int *iters) {
     }
     chem_store(R, m1, a, r, e, rm, re, U);
     return aborted;
-}
-
-// mixture density and internal energy per unit volume exactly as chem_cell forms them
-__device__ __forceinline__ void chem_mixture(const RelaxParams &R, const double *U, double *rm, double *re, double *ag) {
-    const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
-    const double a1 = 1 - a0;
-    const double r0 = U[1] / a0, r1 = U[2] / a1;
-    const double m = a0 * r0 + a1 * r1;
-    const double u = U[3] / m, v = U[4] / m, w = U[5] / m;
-    *rm = m;
-    *re = U[8] - 0.5 * m * (u * u + v * v + w * w);
-    *ag = a1 * r1;
 }
 
 // Full-step Newton from the surrogate's equilibrium (p, T, alpha) on the residuals of chem_system.
@@ -604,9 +609,8 @@ struct InRelax {
         double u[NV];
 #pragma unroll
         for (int v = 0; v < NV; v++) u[v] = U[(size_t)v * n + c];
-        double rm, re, ag;
-        chem_mixture(R, u, &rm, &re, &ag);
-        const float f[3] = {(float)rm, (float)(re / rm), (float)(ag / rm)};
+        const ChemMix m = chem_mixture(R, u);
+        const float f[3] = {(float)m.rm, (float)(m.re / m.rm), (float)(m.ar1 / m.rm)};
 #pragma unroll
         for (int k = 0; k < 3; k++) z[k] = (f[k] - N.xMean[k]) / N.xStd[k];
     }
@@ -662,11 +666,10 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
             double u[NV];
 #pragma unroll
             for (int v = 0; v < NV; v++) u[v] = U[(size_t)v * n + c];
-            double rm, re, ag;
-            chem_mixture(R, u, &rm, &re, &ag);
+            const ChemMix mix = chem_mixture(R, u);
             const float4 p4 = pred[i];
             const float pr[4] = {p4.x, p4.y, p4.z, p4.w};
-            used = chem_polish(R, u, pr, rm, re, S.relTol, S.polishIters, &pits);
+            used = chem_polish(R, u, pr, mix.rm, mix.re, S.relTol, S.polishIters, &pits);
             if (used) {
                 U[(size_t)0 * n + c] = u[0];
                 U[(size_t)1 * n + c] = u[1];
@@ -716,7 +719,12 @@ __global__ void __launch_bounds__(128, kWide ? kWideBlocks : kOrd ? ((kSG && !kP
     if (act && !used) {
 #pragma unroll
         for (int v = 0; v < NV; v++) u[v] = U[(size_t)v * n + c];
-        if (chem && (kPolish || kLog)) chem_mixture(R, u, &rm, &re, &ag);
+        if (chem && (kPolish || kLog)) {
+            const ChemMix mix = chem_mixture(R, u);
+            rm = mix.rm;
+            re = mix.re;
+            ag = mix.ar1;
+        }
         // the network's prediction for this cell (k_sg_tc over the chemical cells) if its input
         // is inside the training hull
         if (kPolish && chem && hullOk[i] != 0) {

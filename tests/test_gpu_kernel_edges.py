@@ -112,6 +112,50 @@ def test_relaxation_kernels_agree_bitwise():
         s.close()
 
 
+def _relaxed(mesh, c, prec, U, log=False):
+    """State after one relaxation, and the residual of it, which shows the primitive records bit for bit."""
+    s = Solver(mesh, c, precision=prec)
+    s.set_state(U)
+    if log:
+        s.relax_log(1_000_000)
+    n = s.relaxation()["nChem"]
+    V = s.get_state()
+    R = None
+    if mesh.n_owned == mesh.n_elem:
+        s.compute_rhs()
+        R = s.get_rhs()
+    s.close()
+    return V, R, n
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("pinf_gas", [0.0, 2e5])
+@pytest.mark.parametrize("vel", [0.0, 25.0])
+def test_every_relaxation_kernel_gives_the_same_states(prec, pinf_gas, vel):
+    """The kernels of few and of many cells, with and without the sample log, and (where no cell is chemical) the one
+    without the chemical branch: the same states and primitive records bit for bit."""
+    nm = meshgen.box_hexes(39, 39, 38, L=(39e-3, 39e-3, 38e-3))
+    m = Mesh.build(nm.nodes, nm.elems, nm.bcs)
+    c = cases.reference_case()
+    c.pInf[1] = pinf_gas
+    U = cases.perturbed_two_phase_ic(c, m.arrays()["cellCenter"], seed=4, vel=vel)
+    whole, R, n = _relaxed(m, c, prec, U)
+    assert n > 1000
+    V, Q, _ = _relaxed(m, c, prec, U, log=True)
+    assert np.array_equal(V, whole) and np.array_equal(Q, R)
+    for p in range(2):
+        part = m.partition(2, p)
+        own = part.partition_maps()["cell_global"][:part.n_owned]
+        V, _, _ = _relaxed(part, c, prec, U[own])
+        assert np.array_equal(V, whole[own])
+    c.chemLimit = 1.0   # no cell is above it
+    whole, R, n = _relaxed(m, c, prec, U)
+    assert n == 0
+    c.chemFlag = 0
+    V, Q, _ = _relaxed(m, c, prec, U)
+    assert np.array_equal(V, whole) and np.array_equal(Q, R)
+
+
 # a tile holds 32 samples, a pass over the blocks 296 tiles
 @pytest.mark.parametrize("n", [1, 31, 33, 296 * 32 + 1])
 def test_training_gradient_batch_sizes(n):
