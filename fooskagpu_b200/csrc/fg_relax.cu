@@ -301,9 +301,14 @@ __device__ __forceinline__ void chem_system(const RelaxParams &R, bool m1, doubl
         T[0] = (p[0] + R.pinf[0]) * (R.icvgm1[0] * (m1 ? irp : ir));
         T[1] = (p[1] + R.pinf[1]) * (R.icvgm1[1] * (m1 ? ir : irp));
         ChemLog l;
-        const double d0 = (T[0] - S.T[0]) * S.iT[0], d1 = (T[1] - S.T[1]) * S.iT[1];
-        const double d2 = (p[0] - S.p[0]) * S.iP[0], d3 = (p[1] - S.p[1]) * S.iP[1];
-        if (q && fabs(d0) < kSmallLog && fabs(d1) < kSmallLog && fabs(d2) < kSmallLog && fabs(d3) < kSmallLog) {
+        double d0 = 1, d1 = 1, d2 = 1, d3 = 1;   // the base point takes logarithms of its own
+        if (q) {
+            d0 = (T[0] - S.T[0]) * S.iT[0];
+            d1 = (T[1] - S.T[1]) * S.iT[1];
+            d2 = (p[0] - S.p[0]) * S.iP[0];
+            d3 = (p[1] - S.p[1]) * S.iP[1];
+        }
+        if (fabs(d0) < kSmallLog && fabs(d1) < kSmallLog && fabs(d2) < kSmallLog && fabs(d3) < kSmallLog) {
             l.lT[0] = log10_1p(d0, S.log.lT[0]);
             l.lT[1] = log10_1p(d1, S.log.lT[1]);
             l.lP[0] = log10_1p(d2, S.log.lP[0]);
