@@ -286,13 +286,20 @@ __global__ void k_field_vars(int n, const double *__restrict__ U, const T *__res
 // automatic surrogate polish pass: a separate pass when fewer than one cell in kSparseChemInv of
 // the previous surrogate relaxation was chemical
 constexpr int kSparseChemInv = 10;
-// most cells of a mesh whose per-cell signal maxima are reset by the CFL kernel (see dt_stage)
-constexpr int kResetCells = 1 << 18;
+// Most cells of a mesh whose per-cell signal maxima are zeroed by the CFL kernel that reads them, for the next dt
+// step; on larger ones a memset does it before the face kernel (see dt_stage).  The memset ends the overlap of the
+// gradient and the face kernel, which costs 3 us whatever the size; but it also brings the array into L2 for the
+// face kernel's atomics, which saves up to 1.5 %.  Step with a new dt, CFL kernel against memset, the same for
+// hexes and tets: mixed 85 k cells 114 / 118 us, 262 k 288 / 290, 373 k 396 / 397, 480 k 402 / 401,
+// 512 k 539 / 537, 885 k 894 / 886, 2.1 M 1997 / 1969; FP64 85 k 282 / 286, 295 k 589.5 / 589.8,
+// 373 k 933.0 / 932.5, 480 k 885 / 881, 2.1 M 4496 / 4450.
+constexpr int kResetCells = 400000;
 
 template <typename T>
 struct SolverT : public fg_solver {
     DevBuf dFlags, dGeo, dVol, dVolP, dIVol, dNew2Old, dHaloStart, dHaloIds, dSlotLocal;
     DevBuf dU, dU0, dRHS, dW[2], dG, dSig, dCellSig, dBlockMin, dScal, dCnt, dCons, dStage;
+    bool cellSigZero = false;   // dCellSig holds zeros (once the work queued so far is done)
     DevBuf dStageIn;   // staging buffer of the asynchronous uploads (on first use)
     DevBuf dStageOut[2];   // staging buffers of the asynchronous downloads (on first use)
     DevBuf dFIdx, dFGeo, dSlotFace, dClosure, dFB;
@@ -622,6 +629,7 @@ struct SolverT : public fg_solver {
         FG_CUDA_TRY(dSig.alloc((size_t)n * sizeof(double)));
         FG_CUDA_TRY(dCellSig.alloc((size_t)n * sizeof(T)));
         FG_CUDA_TRY(cudaMemset(dCellSig.p, 0, (size_t)n * sizeof(T)));
+        cellSigZero = true;
         FG_CUDA_TRY(dBlockMin.alloc((size_t)std::max(flux_blocks(n), cons_blocks(n)) * sizeof(double)));
         FG_CUDA_TRY(dScal.alloc(4 * sizeof(double)));   // dt, time, cons
         FG_CUDA_TRY(dCnt.alloc(8 * sizeof(int32_t)));
@@ -882,13 +890,11 @@ struct SolverT : public fg_solver {
         int rc;
         if ((rc = gradients_halo(s))) return rc;
         Fields<T> f = fields(cur);
-        // Zero maxima before the face kernel: left so by the last dt step's CFL kernel on small meshes, where
-        // a memset between the gradient and the face kernel would end their overlap (8^3 TGV run 290 ->
-        // 272 us, 73,908-tet bubble 979 -> 947, both with the time advance in the gradient kernel); by a memset
-        // on large ones, which also brings the array into L2 for the face kernel's atomics (without it 480 k
-        // tets 9.24 -> 9.36 ms, 2.0 M cells 10.52 -> 10.72 ms; 262 k cells 1806 -> 1794 us).
+        // zero maxima before the face kernel (see kResetCells); a dt step that did not get to its CFL kernel
+        // leaves them to the next one's memset
         const bool reset = n <= kResetCells;
-        if (!reset) FG_CUDA_TRY(cudaMemsetAsync(dCellSig.p, 0, (size_t)n * sizeof(T), s));
+        if (!reset || !cellSigZero) FG_CUDA_TRY(cudaMemsetAsync(dCellSig.p, 0, (size_t)n * sizeof(T), s));
+        cellSigZero = false;
         prof_begin(FG_K_FLUX, s);
         launch_face<T>(dm, f, P, 2, s);
         prof_end(s);
@@ -896,6 +902,7 @@ struct SolverT : public fg_solver {
         launch_cell_cfl<T>(dm, f, reset, s);
         prof_end(s);
         FG_LAUNCH_CHECK("cell cfl");
+        cellSigZero = reset;
         if ((rc = time_step(nullptr, s))) return rc;
         prof_begin(FG_K_GATHER, s);
         launch_gather<T>(dm, f, D, FLUX_FUSED, 0, coef(irk, writeU0), s);

@@ -156,6 +156,28 @@ def test_every_relaxation_kernel_gives_the_same_states(prec, pinf_gas, vel):
     assert np.array_equal(V, whole) and np.array_equal(Q, R)
 
 
+# up to 400,000 cells the CFL kernel leaves the signal maxima at zero, above a memset does
+@pytest.mark.parametrize("nx", [5, 100, 101])
+def test_signal_maxima_start_from_zero(nx):
+    """A dt step after one with faster signals: the new dt is that of the residual path."""
+    nm = meshgen.box_hexes(nx, 100, 40, L=(nx * 1e-2, 1.0, 0.4))
+    m = Mesh.build(nm.nodes, nm.elems, nm.bcs, gpu=True)
+    c = cases.sod_case()
+    c.adaptDtItr = c.relaxFlag = 1
+    x = m.arrays()["cellCenter"]
+    z = np.zeros(len(x))
+    a, b = Solver(m, c, precision="mixed"), Solver(m, c, precision="mixed")
+    for speed in (3.0, 0.0):
+        U = cases.prim_to_cons(c, 0.5, z + 1, z + 1, speed * np.sin(9 * x[:, 1]), z, z, z + 1)
+        for s in (a, b):
+            s.set_state(U)
+        a.step()
+        b.compute_rhs(want_signal=True)
+        assert a.time()[0] == b.compute_time_step()
+    a.close()
+    b.close()
+
+
 # a tile holds 32 samples, a pass over the blocks 296 tiles
 @pytest.mark.parametrize("n", [1, 31, 33, 296 * 32 + 1])
 def test_training_gradient_batch_sizes(n):
