@@ -15,11 +15,7 @@
 //              (DP/update.cu:19-103), or stores the residual.
 #include "fg_kernels.cuh"
 
-#include <climits>
-
-
 namespace fg {
-
 
 // Face records (FREC values).  FP32: 48 consecutive bytes per face, three 16-byte vectors.  FP64: planes
 // of 16-byte vectors as the cell records: 96 consecutive bytes per face made every store and load

@@ -39,14 +39,10 @@ struct DevMesh {
     int nFEval;         // faces the face kernel evaluates (those touching an own cell) come first
     int nSlots;         // slots per cell: 4 (tets only) or 6
     const int32_t *flags; // bits 0-2: faces of the cell; bit 3+k: cell owns the face of slot k
-    // the six per-slot geometry arrays below are consecutive blocks of geoStride values, in this
-    // order, starting at aox; geoStride >= n * nSlots is a multiple of 16 bytes so that every
-    // component starts 16-byte aligned and 16-byte reads of a block's range stay inside it
-    size_t geoStride;
+    // per-slot geometry; every array starts 16-byte aligned, so that a pair of slots is one load
     const T *aox, *aoy, *aoz;        // outward area vector of the slot's face seen from the cell, n A
     const T *dcx, *dcy, *dcz;        // face centre - own cell centre
-    const double *vol;               // cell volume
-    const double *ivol;              // 1 / vol
+    const double *ivol;              // 1 / cell volume
     const double *volP;              // pow(vol, 0.3333) as the reference's CFL bound uses
     // shared-memory staging: blocks of `blockCells` consecutive cells; the face neighbours of a
     // block that lie outside it (its halo) are listed in haloIds[haloStart[b] .. haloStart[b+1]);
@@ -60,7 +56,6 @@ struct DevMesh {
     // ---- faces (each evaluated once by k_face), in tiles of kFaceTile lower cells: by the lower cell's
     //      slot, then by lower cell within a tile ----
     int nF;
-    size_t fStride;                  // component stride of the face geometry arrays
     const uint32_t *fLo;             // lower cell (the smaller index); bit 31: the other one is the owner
     const int32_t *fHi;              // upper cell, or -bc on a boundary face (whose lower cell is the owner)
     const T *fnx, *fny, *fnz, *fA;   // canonical unit normal (owner -> neighbour) and area

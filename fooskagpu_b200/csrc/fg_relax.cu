@@ -76,9 +76,9 @@ __device__ double sat_temp(const RelaxParams &R, double P, double temp, double u
 // operations 23): with s = part_minor / r the primary density is part / (1 - s), so its reciprocal needs
 // none; the stepped density is r (1 + 1e-4), so 1 / r and s scale by a constant; and the Newton step is
 // solved for in units of the difference steps, so the Jacobian's columns stay differences.
-// Bound by FP64 instructions.  981 k-tet bubble (8.6 iterations per cell): 255 us in the reference's order,
-// 159 with shared denominators (11 divisions), 113 now; 2.0 M-cell jet 241, 145, 116; 128^3 TGV (one
-// iteration) 141, 112, 111.
+// Bound by the latency of FP64 instructions (their pipe is 33-53 % busy, see the relaxation's profile).  981 k-tet
+// bubble (8.6 iterations per cell): 255 us in the reference's order, 159 with shared denominators (11
+// divisions), 113 now; 2.0 M-cell jet 241, 145, 116; 128^3 TGV (one iteration) 141, 112, 111.
 __device__ int therm_cell(const RelaxParams &R, double *U, int *iters) {
     const double a0 = fmin(fmax(R.avfMin / 100, U[0]), 1 - R.avfMin / 100);
     const double a1 = 1 - a0;
@@ -595,12 +595,6 @@ __global__ void k_relax_order(int n, const uint8_t *isChem, const int32_t *block
     else order[*total + (b * kOrdThreads - blockOff[b]) + rankT] = c;
 }
 
-
-// kSG / kLog: instantiated with the surrogate path / the solve log; the plain instantiation
-// carries none of their code (and none of their registers).  kPass (with kSG): the surrogate's
-// polish ran before, in k_relax_polish, and the cells it accepted are skipped; otherwise the
-// polish runs here.  kOrd: thread i relaxes cell order[i], chemical when i < *nChem
-// (k_relax_order); otherwise thread i relaxes cell i and decides the branch itself.
 // surrogate input of the relaxation: chemical cell order[i], i < *nChem
 struct InRelax {
     const double *U;
@@ -699,6 +693,11 @@ __global__ void __launch_bounds__(128, FG_CHEM_SG_MINBLOCKS) k_relax_polish(int 
     }
 }
 
+// kSG / kLog: instantiated with the surrogate path / the solve log; the plain instantiation
+// carries none of their code (and none of their registers).  kPass (with kSG): the surrogate's
+// polish ran before, in k_relax_polish, and the cells it accepted are skipped; otherwise the
+// polish runs here.  kOrd: thread i relaxes cell order[i], chemical when i < *nChem
+// (k_relax_order); otherwise thread i relaxes cell i, thermally.
 template <typename T, bool kSG, bool kLog, bool kOrd, bool kPass = false, bool kWide = false>
 __global__ void __launch_bounds__(128, kWide ? kWideBlocks : kOrd ? ((kSG && !kPass) ? FG_CHEM_SG_MINBLOCKS : FG_CHEM_MINBLOCKS)
                                             : FG_THERM_MINBLOCKS) k_relax(int n, double *U, T *W, size_t wStride, const PhysD D, const RelaxParams R,

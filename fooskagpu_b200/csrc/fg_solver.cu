@@ -432,7 +432,7 @@ struct SolverT : public fg_solver {
             }
         }
         const size_t S = (size_t)nSlots * n;
-        // component stride of the geometry arrays: padded to 16 bytes (see DevMesh::geoStride)
+        // component stride of the geometry arrays: padded to 16 bytes, as the kernels load pairs
         const size_t GS = (S * sizeof(T) + 15) / 16 * 16 / sizeof(T);
         std::vector<int32_t> nbr(S, INT32_MIN), flags(n, 0);
         std::vector<T> geo(6 * GS, (T)0);
@@ -664,14 +664,11 @@ struct SolverT : public fg_solver {
         dm.nSlots = nSlots;
         dm.flags = dFlags.as<int32_t>();
         T *g = dGeo.as<T>();
-        dm.geoStride = GS;
         dm.aox = g + 0 * GS; dm.aoy = g + 1 * GS; dm.aoz = g + 2 * GS;
         dm.dcx = g + 3 * GS; dm.dcy = g + 4 * GS; dm.dcz = g + 5 * GS;
-        dm.vol = dVol.as<double>();
         dm.ivol = dIVol.as<double>();
         dm.volP = dVolP.as<double>();
         dm.nF = nF;
-        dm.fStride = FS;
         {
             const T *fg = dFGeo.as<T>();
             dm.fnx = fg; dm.fny = fg + FS; dm.fnz = fg + 2 * FS; dm.fA = fg + 3 * FS;

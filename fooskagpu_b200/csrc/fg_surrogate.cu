@@ -57,17 +57,19 @@ struct Buf {
 // ---- one training pass over a batch: forward, loss, backward and weight gradients in one kernel,
 // then a reduction over its blocks with the Adam step.
 //
-// A block of 256 threads takes tiles of kTrainS samples (grid-stride, kTrainS small enough that a
-// 4096-sample batch fills the SMs), keeps the parameters and the tile's activations in shared
-// memory, and accumulates its share of every weight gradient in registers over its tiles; the
-// block's sums go to part[block][SG_NPARAM] once, at the end.  Bound by FP32 multiply-adds from
-// shared memory (26 k per sample): a thread computes 2 samples x 4 outputs of a layer (one 16-byte
-// read of a weight row feeds 8 multiply-adds), 4 x 4 of a weight gradient.  Rows have a pitch of 68
-// values, so that 8 lanes reading 16 bytes of 8 consecutive rows hit distinct banks.
+// A block of 256 threads takes tiles of kTrainS samples (grid-stride), keeps the parameters and the
+// tile's activations in shared memory, and accumulates its share of every weight gradient in registers
+// over its tiles; the block's sums go to part[block][SG_NPARAM] once, at the end.  A thread computes
+// 2 samples x 4 outputs of a layer (one 16-byte read of a weight row feeds 8 multiply-adds), 4 x 4 of a
+// weight gradient.  Rows have a pitch of 68 values, so that 8 lanes reading 16 bytes of 8 consecutive rows
+// hit distinct banks.  Up to 4096 samples (128 blocks, one on each of 128 SMs, 20 SMs idle) the time is
+// that of one tile's chain of layers: 15.4 us for 64 samples, 15.9 for 512, 16.7 for 4096, 12.7 of the
+// 74 TFLOP/s.  Where every block slot is taken it is bound by FP32 multiply-adds from shared memory (26 k
+// per sample): 9,472 samples 25.8 us, 16,384 44.6, 131,072 274 us, 25 TFLOP/s.
 // Summation order: a block's samples in order, then the blocks in a fixed order, so training is
 // deterministic for a given batch size.
-// Measured (B200, batch 4096): 17.9 us, and 3 us for the reduction, against 230 us for the 15 launches of
-// one layer or one reduction each that it replaced; an epoch of 16 batches 4.44 -> 0.70 ms.
+// Batch 4096: 16.7 us, and 3 us for the reduction, against 230 us for the 15 launches of one layer or one
+// reduction each that it replaced; an epoch of 16 batches 4.44 -> 0.70 ms.
 constexpr int kTrainS = 32, kTrainThreads = 256, kTrainPitch = SG_H + 4;
 constexpr int kTrainMaxBlocks = 296;   // 2 resident blocks on each of 148 SMs
 constexpr int kTrainRows = kTrainS * kTrainPitch;
